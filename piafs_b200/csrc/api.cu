@@ -155,7 +155,7 @@ static void enqueue_rhs(piafs_gpu_sim* s, double* rhs, const double* U, const do
 }
 
 void piafs::enqueue_bc(piafs_gpu_sim* s, double* u) {
-  for (const Zone& z : s->deck.zones) launch_bc(s->P, u, z, s->stream);
+  launch_bc(s->P, u, s->deck.zones.data(), (int)s->deck.zones.size(), s->stream);
 }
 
 // One time step: TimePreStep's boundary conditions on u, TimeRK's stages and
@@ -391,10 +391,10 @@ int piafs_gpu_get_info(piafs_gpu_sim* s, piafs_gpu_info* info) {
   info->npoints_ghosted = s->P.npg;
   info->ninterfaces[0] = s->P.nint[0]; info->ninterfaces[1] = s->P.nint[1];
   info->cfl = s->last_cfl; info->norm = s->last_norm; info->singular = s->singular;
-  // kernels per step: prestep BCs, per stage (combine + BCs for s > 0, flux
+  // kernels per step: the prestep BC launches (nz), per stage (combine + BCs for s > 0, flux
   // and reconstruction per direction plus the transpose of a transposed y
   // pass, one upwind/divergence kernel, viscous/source), update, clock
-  const int nz = (int)d.zones.size();
+  const int nz = launch_bc(s->P, nullptr, d.zones.data(), (int)d.zones.size(), nullptr);
   const int vs = ((s->P.ndims == 2 && s->P.viscous) || s->P.chem) ? 1 : 0;
   const int tr = (s->ut && s->P.model != NS2D) ? 1 : 0;   // NS2D: the transpose also forms the y flux
   info->launches_per_step = nz + d.nstages * (2 * s->P.ndims + 1 + tr + vs) + (d.nstages - 1) * (1 + nz) + 2;

@@ -33,32 +33,45 @@ struct Zone {
 };
 
 #ifdef __CUDACC__
+// zone types whose ghosts are a function of one variable at one point
+// (every variable alike), and that value at source point p2
+__host__ __device__ __forceinline__ bool bc_per_variable(int type) {
+  return type == BC_PERIODIC || type == BC_EXTRAPOLATE || type == BC_DIRICHLET || type == BC_REFLECT;
+}
+__device__ __forceinline__ double bc_variable(const DevParams& P, const Zone& z, const double* u, long long p2,
+                                              int v) {
+  if (z.type == BC_DIRICHLET) return z.val[v];                        // BCDirichlet.c:26-39
+  const double x = u[v * P.ps + p2];
+  return z.type == BC_REFLECT ? -1.0 * x : x;                         // BCReflect.c:27-50
+}
+// The source point of ghost (g0, g1).  The periodic source keeps the
+// zone-relative index in the other dimension, as the reference does.
+__device__ __forceinline__ long long bc_source(const DevParams& P, const Zone& z, int g0, int g1) {
+  const int d = z.dim, b = (d == 0 ? g0 : g1) - z.is[d];
+  int src[2] = {g0, g1};
+  const int Nd = d == 0 ? P.N0 : P.N1;
+  if (z.type == BC_PERIODIC) {
+    if (P.ndims == 2) src[1 - d] = src[1 - d] - z.is[1 - d];
+    src[d] = z.face == 1 ? b + Nd - P.ghosts : b;
+  } else {
+    src[d] = z.face == 1 ? P.ghosts - 1 - b : Nd - b - 1;
+  }
+  return pidx(P, src[0], src[1]);
+}
+
 // Boundary values at ghost point (g0, g1) of zone z (BCPeriodic.c,
 // BCExtrapolate.c, BCSlipWall.c and the boundaries below): reads the zone's
 // source point of u (SoA planes) and writes the ghost's variables to
 // out[v * ostride] -- all of them, or for the flow boundaries of the
 // Euler / Navier-Stokes models the flow variables (and the passive scalars
-// of an inflow) only; the others stay untouched.  The periodic source keeps the zone-relative index in
-// the other dimension, as the reference does.
+// of an inflow) only; the others stay untouched.
 __device__ __forceinline__ void bc_point(const DevParams& P, const Zone& z, const double* u, int g0, int g1,
                                          double* out, long long ostride) {
-  const int gi[2] = {g0, g1};
-  const int d = z.dim, b = gi[d] - z.is[d];
-  int src[2] = {g0, g1};
+  const int d = z.dim;
   const int Nd = d == 0 ? P.N0 : P.N1;
-  if (z.type == BC_PERIODIC) {
-    if (P.ndims == 2) src[1 - d] = gi[1 - d] - z.is[1 - d];
-    src[d] = z.face == 1 ? b + Nd - P.ghosts : b;
-  } else {
-    src[d] = z.face == 1 ? P.ghosts - 1 - b : Nd - b - 1;
-  }
-  const long long p2 = pidx(P, src[0], src[1]);
-  if (z.type == BC_DIRICHLET) {        // BCDirichlet.c:26-39
-    for (int v = 0; v < P.nvars; v++) out[v * ostride] = z.val[v];
-    return;
-  }
-  if (z.type == BC_REFLECT) {          // BCReflect.c:27-50
-    for (int v = 0; v < P.nvars; v++) out[v * ostride] = -1.0 * u[v * P.ps + p2];
+  const long long p2 = bc_source(P, z, g0, g1);
+  if (bc_per_variable(z.type)) {
+    for (int v = 0; v < P.nvars; v++) out[v * ostride] = bc_variable(P, z, u, p2, v);
     return;
   }
   if (z.type >= BC_NOSLIP) {
@@ -125,8 +138,6 @@ __device__ __forceinline__ void bc_point(const DevParams& P, const Zone& z, cons
       out[2 * ostride] = rho * vg;
       out[3 * ostride] = igm1 * pr + 0.5 * rho * (ug * ug + vg * vg);
     }
-  } else {
-    for (int v = 0; v < P.nvars; v++) out[v * ostride] = u[v * P.ps + p2];
   }
 }
 #endif
@@ -137,7 +148,9 @@ void launch_soa_to_interior(const DevParams& P, const double* soa, double* out, 
 void launch_interior_to_soa(const DevParams& P, const double* in, double* soa, cudaStream_t s);
 void launch_iface_aos_to_soa(const double* aos, double* soa, long long ni, int nv, long long pis, cudaStream_t s);
 void launch_iface_soa_to_aos(const double* soa, double* aos, long long ni, int nv, long long pis, cudaStream_t s);
-void launch_bc(const DevParams& P, double* u, const Zone& z, cudaStream_t s);
+// the deck's boundary zones applied to the ghosts of u, in the deck's order;
+// returns the number of launches (u null: counted, not launched)
+int launch_bc(const DevParams& P, double* u, const Zone* z, int nz, cudaStream_t s);
 // 2D only: plane-wise transpose of a ghosted state (j fastest in `out`) and
 // the parameters that describe the transposed grid (dimensions swapped)
 void launch_transpose(const DevParams& P, const double* in, double* out, cudaStream_t s);
