@@ -77,27 +77,34 @@ __global__ void __launch_bounds__(line_threads_max(), 1)
   int bad = 0;
   line_pair_solve<M, WT, R, O>(P, src, st, ref, N, cs, pcA, tp, sy, so, bad);
   if (bad) atomicOr(err, 1);
-  const int ostride = opad(N) + 1;
   // N + 1 interfaces over Pt threads: at most M + 1 each; the passive
   // variables packed for their upwinding when P.pack_sp (uL - uR, fL + fR)
+  const O* o = so + padm<M>(k);
+  const int ostride = padm<M>(N) + 1, ostep = Pt + Pt / M;   // Pt is a multiple of M
+  oL += k * ist;
+  oR += k * ist;
+  const long long gstep = Pt * ist;
   if (P.pack_sp && v >= P.nflow) {
 #pragma unroll
     for (int it = 0; it <= M; it++) {
-      const int i = k + it * Pt;
-      if (i <= N) {
-        const O l = so[opad(i)], r = so[ostride + opad(i)];
-        oL[i * ist] = isF ? l + r : l - r;
+      if (k + it * Pt <= N) {
+        const O l = *o, r = o[ostride];
+        *oL = isF ? l + r : l - r;
       }
+      o += ostep;
+      oL += gstep;
     }
     return;
   }
 #pragma unroll
   for (int it = 0; it <= M; it++) {
-    const int i = k + it * Pt;
-    if (i <= N) {
-      oL[i * ist] = so[opad(i)];
-      oR[i * ist] = so[ostride + opad(i)];
+    if (k + it * Pt <= N) {
+      *oL = *o;
+      *oR = o[ostride];
     }
+    o += ostep;
+    oL += gstep;
+    oR += gstep;
   }
 }
 
@@ -149,9 +156,9 @@ __global__ void __launch_bounds__(line_threads_max(), 1)
   const int kN = (N - 2) / M;                // separator owning row N-1
   const R eps = R(4) * (R)P.eps;
   int bad = 0;
-  // cells rb-3 .. rb+Pt M+2 at staged index j = cell - rb + 3, zero past N+2
+  // cells rb-3 .. rb+Pt M+3 at staged index j = cell - rb + 3, zero past N+2
   {
-    const int ncell = Pt * M + 6;
+    const int ncell = Pt * M + 7;
     double cv[M + 1];
 #pragma unroll
     for (int it = 0; it <= M; it++) {
@@ -161,23 +168,18 @@ __global__ void __launch_bounds__(line_threads_max(), 1)
 #pragma unroll
     for (int it = 0; it <= M; it++) {
       const int j = k + it * Pt;
-      if (j < ncell) cs[cpad(j)] = cv[it];
+      if (j < ncell) cs[padm<M>(j)] = cv[it];
     }
   }
-  double x0[2] = {0.0, 0.0}, xN[2] = {0.0, 0.0};
-  if (MX) {
-    if (K == 0) { x0[0] = crw_edge_f(P, src, st, 0, 1, ref); x0[1] = crw_edge_f(P, src, st, 0, -1, ref); }
-    if (K == kN) { xN[0] = crw_edge_f(P, src, st, N, 1, ref); xN[1] = crw_edge_f(P, src, st, N, -1, ref); }
-  } else {
-    if (K == 0) { x0[0] = crw_edge(P, src, st, 0, 1); x0[1] = crw_edge(P, src, st, 0, -1); }
-    if (K == kN) { xN[0] = crw_edge(P, src, st, N, 1); xN[1] = crw_edge(P, src, st, N, -1); }
-  }
   __syncthreads();
+  double x0[2] = {0.0, 0.0}, xN[2] = {0.0, 0.0};
+  const int Kw = K - lane;                   // first separator of this warp
+  if (Kw == 0 || Kw == kN - (kN & 31))       // warps start at multiples of 32: Pt is one
+    crw_edges<M, WT, R>(P, cs, Kw == 0 ? 0 : N - rb, Kw == kN - (kN & 31) ? N - rb : 0, x0, xN);
 
   double As[2], Bs[2], Cs[2], Rs[2];
   double al[2][M], cg_[2][M], rh[2][M];
-  const int Kw = K - lane;                   // first separator of this warp
-  if (Kw >= 1 && (Kw + 32) * M <= N - 2)
+  if ((Kw + 32) * M <= N - 2)
     crw_chunk<M, WT, true, R>(cs, k, s, N, x0, xN, eps, As, Bs, Cs, Rs, al, cg_, rh, bad);
   else
     crw_chunk<M, WT, false, R>(cs, k, s, N, x0, xN, eps, As, Bs, Cs, Rs, al, cg_, rh, bad);
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(line_threads_max(), 1)
   // separator equations, scaled to a unit diagonal; the first separator of
   // CTA r > 0 couples to the previous CTA's last one (L, column e) and the
   // last of CTA r < ncta-1 to the next CTA's first (R, column f)
-  double a[2], cq[2], d[2], e[2], f[2];
+  double a[2], cq[2], x[3][2];   // x: the columns d, e, f
   {
     double2 alp = make_double2(0.0, 0.0), gap = alp, rhp = alp;
     if (k > 0) {
@@ -206,50 +208,21 @@ __global__ void __launch_bounds__(line_threads_max(), 1)
       const double rbq = rcp_nr(b);
       a[q] = -(As[q] * alq[q]) * rbq;
       cq[q] = -(Cs[q] * cg_[q][1]) * rbq;
-      d[q] = (Rs[q] - As[q] * rhq[q] - Cs[q] * rh[q][1]) * rbq;
-      e[q] = 0.0;
-      f[q] = 0.0;
-      if (k == 0) { e[q] = a[q]; a[q] = 0.0; }
-      if (k == Pt - 1) { f[q] = cq[q]; cq[q] = 0.0; }
+      x[0][q] = (Rs[q] - As[q] * rhq[q] - Cs[q] * rh[q][1]) * rbq;
+      x[1][q] = 0.0;
+      x[2][q] = 0.0;
+      if (k == 0) { x[1][q] = a[q]; a[q] = 0.0; }
+      if (k == Pt - 1) { x[2][q] = cq[q]; cq[q] = 0.0; }
     }
   }
-  auto put = [&](double2* row) {
-    row[k] = make_double2(a[0], a[1]);
-    row[Pt + k] = make_double2(cq[0], cq[1]);
-    row[2 * Pt + k] = make_double2(d[0], d[1]);
-    row[3 * Pt + k] = make_double2(e[0], e[1]);
-    row[4 * Pt + k] = make_double2(f[0], f[1]);
-  };
-  put(pcA);
-  __syncthreads();
-  // PCR within the CTA (rows outside it: zero couplings, clamped as in
-  // line_pair_solve), the external unknowns' columns updated alongside
-  int buf = 0;
-  for (int dl = 1; dl < Pt; dl <<= 1) {
-    const double2* cur = pcA + buf * 5 * Pt;
-    const int km = k >= dl ? k - dl : k, kp = k + dl < Pt ? k + dl : k;
-    const double2 am = cur[km], cm = cur[Pt + km], dm = cur[2 * Pt + km], em = cur[3 * Pt + km],
-                  fm = cur[4 * Pt + km];
-    const double2 ap = cur[kp], cp = cur[Pt + kp], dp = cur[2 * Pt + kp], ep = cur[3 * Pt + kp],
-                  fp = cur[4 * Pt + kp];
-    const double amq[2] = {am.x, am.y}, cmq[2] = {cm.x, cm.y}, dmq[2] = {dm.x, dm.y}, emq[2] = {em.x, em.y},
-                 fmq[2] = {fm.x, fm.y};
-    const double apq[2] = {ap.x, ap.y}, cpq[2] = {cp.x, cp.y}, dpq[2] = {dp.x, dp.y}, epq[2] = {ep.x, ep.y},
-                 fpq[2] = {fp.x, fp.y};
+  pcA[k] = make_double2(a[0], a[1]);
+  pcA[Pt + k] = make_double2(cq[0], cq[1]);
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
-      const double bn = 1.0 - a[q] * cmq[q] - cq[q] * apq[q];
-      const double rbq = rcp_nr(bn);
-      const double an = -(a[q] * amq[q]) * rbq, cn = -(cq[q] * cpq[q]) * rbq;
-      d[q] = (d[q] - a[q] * dmq[q] - cq[q] * dpq[q]) * rbq;
-      e[q] = (e[q] - a[q] * emq[q] - cq[q] * epq[q]) * rbq;
-      f[q] = (f[q] - a[q] * fmq[q] - cq[q] * fpq[q]) * rbq;
-      a[q] = an; cq[q] = cn;
-    }
-    put(pcA + (buf ^ 1) * 5 * Pt);
-    buf ^= 1;
-    __syncthreads();
-  }
+  for (int n = 0; n < 3; n++) pcA[(2 + n) * Pt + k] = make_double2(x[n][0], x[n][1]);
+  __syncthreads();
+  // PCR within the CTA, the external unknowns' columns reduced alongside
+  crw_pcr<5>(pcA, Pt, k, a, cq, x);
+  double (&d)[2] = x[0], (&e)[2] = x[1], (&f)[2] = x[2];
   // X_k = d_k - e_k L - f_k R; the first and last rows to the cluster
   if (k == 0) { bnd[0] = make_double2(d[0], d[1]); bnd[1] = make_double2(e[0], e[1]); bnd[2] = make_double2(f[0], f[1]); }
   if (k == Pt - 1) { bnd[3] = make_double2(d[0], d[1]); bnd[4] = make_double2(e[0], e[1]); bnd[5] = make_double2(f[0], f[1]); }
@@ -309,27 +282,25 @@ __global__ void __launch_bounds__(line_threads_max(), 1)
     cg_[0][M - 1] = l1.x; cg_[1][M - 1] = l1.y;
     rh[0][M - 1] = l2.x; rh[1][M - 1] = l2.y;
   }
-  const int ostride = opad(Pt * M + 1) + 1;
+  const int ostride = padm<M>(Pt * M + 1) + 1;
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     const double Xk = d[q], Xn = q == 0 ? xn.x : xn.y;
-    O* o = so + q * ostride;
-    if (s <= N - 1) o[opad(s - rb)] = (O)Xk;
+    O* o = so + q * ostride + k * (M + 1);   // row s + r at padm<M>(1 + r)
+    if (s <= N - 1) o[padm<M>(1)] = (O)Xk;
 #pragma unroll
-    for (int r = 1; r < M; r++) {
-      const int i = s + r;
-      if (i <= N - 1) o[opad(i - rb)] = (O)(rh[q][r] - al[q][r] * Xk - cg_[q][r] * Xn);
-    }
-    if (K == 0) o[0] = (O)x0[q];
-    if (K == kN) o[opad(N - rb)] = (O)xN[q];
+    for (int r = 1; r < M; r++)
+      if (s + r <= N - 1) o[padm<M>(1 + r)] = (O)(rh[q][r] - al[q][r] * Xk - cg_[q][r] * Xn);
+    if (K == 0) so[q * ostride] = (O)x0[q];
+    if (K == kN) so[q * ostride + padm<M>(N - rb)] = (O)xN[q];
   }
   if (bad) atomicOr(err, 1);
   __syncthreads();
   const int lo = rank == 0 ? 0 : rb + 1;
   const int hi = kN / Pt == rank ? N : min(N - 1, rb + Pt * M);
   for (int i = lo + k; i <= hi; i += Pt) {
-    oL[i * ist] = so[opad(i - rb)];
-    oR[i * ist] = so[ostride + opad(i - rb)];
+    oL[i * ist] = so[padm<M>(i - rb)];
+    oR[i * ist] = so[ostride + padm<M>(i - rb)];
   }
 }
 
@@ -338,17 +309,17 @@ __global__ void __launch_bounds__(line_threads_max(), 1)
 template <int M, bool MX>
 size_t line_smem(int N, int Pt) {
   const size_t osz = MX ? sizeof(float) : sizeof(double);
-  const size_t cells = (size_t)(Pt * M + 6 + (Pt * M + 6) / 8 + 1) * sizeof(double);
-  const size_t outs = (size_t)2 * (N + N / 16 + 1) * osz;
+  const size_t cells = (size_t)(padm<M>(Pt * M + 6) + 1) * sizeof(double);
+  const size_t outs = (size_t)2 * (padm<M>(N) + 1) * osz;
   return (size_t)10 * Pt * sizeof(double2) + (cells > outs ? cells : outs);
 }
 
 template <bool MX>
 size_t seg_smem(int Pt) {
   const size_t osz = MX ? sizeof(float) : sizeof(double);
-  const int M = 8;
-  const size_t cells = (size_t)(Pt * M + 6 + (Pt * M + 6) / 8 + 1) * sizeof(double);
-  const size_t outs = (size_t)2 * (opad(Pt * M + 1) + 1) * osz;
+  constexpr int M = 8;
+  const size_t cells = (size_t)(padm<M>(Pt * M + 6) + 1) * sizeof(double);
+  const size_t outs = (size_t)2 * (padm<M>(Pt * M + 1) + 1) * osz;
   return (size_t)(14 * Pt + 8) * sizeof(double2) + (cells > outs ? cells : outs);
 }
 
