@@ -172,7 +172,7 @@ struct piafs_gpu_batch {
   int* dtiles = nullptr;
   int* dntiles = nullptr;
   int tile_cap = 0, ntiles = 0;
-  int shape = 0;                       // index into kShapes
+  int shape = kDefaultShape;           // index into kShapes
   int max_nv = 0, max_stages = 0;
   bool dirty = true;                   // tile list / member table need upload
   cudaGraphExec_t graph = nullptr;

@@ -69,6 +69,8 @@ struct TileShape { int tx, ty, nt, minb; };
 constexpr int kNumShapes = 8;
 constexpr TileShape kShapes[kNumShapes] = {{16, 16, 512, 1}, {32, 8, 512, 1}, {16, 8, 256, 2}, {32, 4, 256, 2},
                                            {8, 16, 256, 2},  {16, 15, 512, 1}, {32, 7, 512, 1}, {16, 7, 256, 2}};
+// where the tuner has not chosen: 16 x 15, whose upwinding is one round
+constexpr int kDefaultShape = 5;
 
 __host__ __device__ constexpr long long al16(long long b) { return (b + 15) / 16 * 16; }
 
@@ -188,6 +190,18 @@ __device__ __noinline__ void iface_upwind_flow(const DevParams& P,
   for (int m = 0; m < NF; m++) so[m * sstride] = fi[m];
 }
 
+// iface_upwind_flow with the deck's scheme (one branch, the same for a whole
+// member: the tile around it is compiled once, not once per scheme)
+template <int MODEL, bool MX, typename... A>
+__device__ __forceinline__ void upwind_by_scheme(const DevParams& P, A... a) {
+  switch (P.upwind) {
+    case UPW_ROE: iface_upwind_flow<MODEL, UPW_ROE, MX>(P, a...); break;
+    case UPW_RF: iface_upwind_flow<MODEL, UPW_RF, MX>(P, a...); break;
+    case UPW_LLF: iface_upwind_flow<MODEL, UPW_LLF, MX>(P, a...); break;
+    default: iface_upwind_flow<MODEL, UPW_RUSANOV, MX>(P, a...); break;
+  }
+}
+
 // the Runge-Kutta part of stage s at point p with stage derivatives k
 __device__ __forceinline__ void rk_point(const BMember& M, const BState& Sd, int s, long long p, int nv) {
   const long long ps = M.P.ps;
@@ -219,12 +233,20 @@ __device__ __forceinline__ void rk_point(const BMember& M, const BState& Sd, int
 //            the fly)
 //   fluxes   flow-variable fluxes and the normal velocity at every stencil
 //            cell of either direction
-//   WENO     WENO5 values of the flow variables, item = (interface, var)
+//   WENO     WENO5 values of the flow variables, item = (field, var, strip of
+//            at most nine interfaces of a line)
 //   upwind   characteristic/scalar upwinding, item = interface
 //   passive  WENO5 + scalar upwinding of a passive variable (flux vn u_m),
-//            item = (interface, var)
+//            item = (var, strip)
 //   viscous  Q, viscous face fluxes (k_visc_source on the tile)
 //   point    stage derivative, chemistry, Runge-Kutta combination
+// The tile is bound by FP64 issue and by the latency of its phases at 16 warps
+// an SM.  Interface by interface the reconstruction took 92 operations a field
+// and pair of biases and read every cell six times; in strips
+// (weno5_strip_js) it takes 46 and reads it once: a stage of twelve 64^2 .. 256^2
+// members went from 271 us (16 x 16 tiles) to 191, to 179 with 16 x 15 tiles, the
+// default, whose interfaces are one round of the upwinding; a mixed-
+// precision serving job of 40 steps from 20.0 to 16.6 ms.
 // Interfaces are numbered x first (f < NXI: row jj, position ii) then y
 // (row jj, column ii), x fastest in both.
 // Shared memory (bytes, regions 16-byte aligned): sU [nv][HY][HX] (FP64);
@@ -242,9 +264,17 @@ __device__ __forceinline__ void rk_point(const BMember& M, const BState& Sd, int
 template <int TX, int TY, bool MX>
 struct Tile2D {
   typedef typename std::conditional<MX, float, double>::type T;
-  static constexpr int HX = TX + 6, HY = TY + 6;
+  // HX: the pitch of a row of TX + 6 cells, odd so that threads on different
+  // rows read different banks
+  static constexpr int HX = (TX + 6) | 1, HY = TY + 6;
   static constexpr int NXI = TY * (TX + 1), NYI = TX * (TY + 1), NI = NXI + NYI;
   static constexpr int NCX = TY * HX, NCY = TX * HY;            // stencil cells per direction
+  // strips of at most nine consecutive interfaces of a line, one thread's work
+  // in the reconstruction: x lines first (row fastest), then y lines (column
+  // fastest)
+  static constexpr int NSX = (TX + 1 + 8) / 9, SX = (TX + 1 + NSX - 1) / NSX;
+  static constexpr int NSY = (TY + 1 + 8) / 9, SY = (TY + 1 + NSY - 1) / NSY;
+  static constexpr int SMAX = SX > SY ? SX : SY, NSTRX = TY * NSX, NSTR = NSTRX + TX * NSY;
   static constexpr long long VISC =
       al16((3LL * (TY + 2) * (TX + 2) + 3LL * TY * (TX + 1) + 3LL * (TY + 1) * TX) * (long long)sizeof(T));
   static constexpr long long REC = al16(16LL * NI * (long long)sizeof(T));
@@ -297,7 +327,7 @@ __device__ __forceinline__ void chem_source_kv(const DevParams& P, const double*
   kv[3] += (double)Q;
 }
 
-template <int TX, int TY, int UPW, int BT, bool MX>
+template <int TX, int TY, int BT, bool MX>
 __device__ __forceinline__ void tile2d(const BMember& M, const BState& Sd, int s, int tx, int ty, char* smem) {
   typedef Tile2D<TX, TY, MX> L;
   typedef typename L::T T;
@@ -322,7 +352,11 @@ __device__ __forceinline__ void tile2d(const BMember& M, const BState& Sd, int s
   int* spm = (int*)((char*)spa + L::SPA);                // [NI]
   const int tid = threadIdx.x;
   constexpr int c0 = H * HX + H;                         // the tile's first interior cell
-  for (int e = tid; e < vs; e += BT) load_point(M, S, i0 - H + e % HX, j0 - H + e / HX, sU + e, vs);
+  constexpr int WX = TX + 2 * H;                         // cells of a row (its pitch is HX)
+  for (int e = tid; e < WX * HY; e += BT) {
+    const int a = e % WX, b = e / WX;
+    load_point(M, S, i0 - H + a, j0 - H + b, sU + b * HX + a, vs);
+  }
   __syncthreads();
   // cell data: x cells (row jj, column a): c = (jj+H)*HX + a, index jj*HX + a;
   // y cells (row b, column ii): c = b*HX + ii + H, index b*TX + ii
@@ -330,7 +364,10 @@ __device__ __forceinline__ void tile2d(const BMember& M, const BState& Sd, int s
     double fr0[4], fr1[4], vr0, vr1;                     // reference fluxes (x, y) at c0
     ns2d_flux(sU[c0], sU[vs + c0], sU[2 * vs + c0], sU[3 * vs + c0], P.gamma, 0, fr0, vr0);
     ns2d_flux(sU[c0], sU[vs + c0], sU[2 * vs + c0], sU[3 * vs + c0], P.gamma, 1, fr1, vr1);
-    for (int e = tid; e < nv * vs; e += BT) sUf[e] = (float)(sU[e] - sU[(e / vs) * vs + c0]);
+    for (int m = 0; m < nv; m++) {
+      const double ref = sU[m * vs + c0];
+      for (int e = tid; e < vs; e += BT) sUf[m * vs + e] = (float)(sU[m * vs + e] - ref);
+    }
     for (int e = tid; e < NCX + NCY; e += BT) {
       const bool xd = e < NCX;
       const int g = xd ? e : e - NCX;
@@ -361,97 +398,112 @@ __device__ __forceinline__ void tile2d(const BMember& M, const BState& Sd, int s
     }
   }
   __syncthreads();
-  // geometry of interface f: its cell i (right of the interface) in sU
-  // (base, stride ust along the line), in its direction's cell data (index
-  // cdo, plane cst, stride cls along the line) and whether it is inside the
-  // member.  Consecutive interfaces of either direction are consecutive in x,
-  // so a warp's shared-memory accesses are unit-stride.
-  auto geo = [&](int f, int& base, int& ust, int& cdo, int& cst, int& cls, int& dir) -> bool {
+  // geometry of interface f: its cell i (right of the interface) in sU and its
+  // stride along the line, and whether it is inside the member
+  auto geo = [&](int f, int& base, int& ust, int& dir) -> bool {
     if (f < NXI) {
       const int ii = f % (TX + 1), jj = f / (TX + 1);
-      base = (jj + H) * HX + ii + H; ust = 1; cdo = jj * HX + ii + H; cst = NCX; cls = 1; dir = 0;
+      base = (jj + H) * HX + ii + H; ust = 1; dir = 0;
       return i0 + ii <= N0 && j0 + jj < N1;
     }
     const int g = f - NXI, ii = g % TX, jj = g / TX;
-    base = (jj + H) * HX + ii + H; ust = HX; cdo = (jj + H) * TX + ii; cst = NCY; cls = TX; dir = 1;
+    base = (jj + H) * HX + ii + H; ust = HX; dir = 1;
     return j0 + jj <= N1 && i0 + ii < N0;
   };
-  // a thread takes NW items at a time and finishes them together (their loads
-  // and arithmetic are independent, so their latencies overlap); items past
-  // the end or outside the member are computed on in-tile data and dropped
-  constexpr int NW = 2;
-  auto load_stencil = [&](int m, int base, int ust, int cdo, int cst, int cls, int dir, T* a, T* b) {
-    if constexpr (MX) {
-      const float* u = sUf + m * vs + base;
-      const float* fc = (dir ? cyf : cxf) + m * cst + cdo;
-#pragma unroll
-      for (int r = 0; r < 6; r++) { a[r] = u[(r - 3) * ust]; b[r] = fc[(r - 3) * cls]; }
-    } else {
-      const double* u = sU + m * vs + base;
-      if (m < 4) {
-        const double* fc = (dir ? cy : cx) + m * cst + cdo;
-#pragma unroll
-        for (int r = 0; r < 6; r++) { a[r] = u[(r - 3) * ust]; b[r] = fc[(r - 3) * cls]; }
-      } else {
-        const double* vn = (dir ? cy : cx) + 4 * cst + cdo;
-#pragma unroll
-        for (int r = 0; r < 6; r++) { a[r] = u[(r - 3) * ust]; b[r] = __dmul_rn(vn[(r - 3) * cls], a[r]); }
-      }
+  // geometry of strip q: its first stencil cell (three left of its first
+  // interface's right cell) in sU and in its direction's cell data, strides
+  // along the line, its first interface, their stride and number.  Threads of
+  // a warp work on neighbouring lines, at the same place along them.
+  struct Strip { int u, us, f, fs, dir, i, is, n; };
+  auto strip = [&](int q) -> Strip {
+    if (q < L::NSTRX) {
+      const int jj = q % TY, p0 = q / TY * L::SX;
+      return {(jj + H) * HX + p0, 1, jj * HX + p0, 1, 0, jj * (TX + 1) + p0, 1, min(L::SX, TX + 1 - p0)};
     }
+    const int g = q - L::NSTRX, ii = g % TX, p0 = g / TX * L::SY;
+    return {p0 * HX + ii + H, HX, p0 * TX + ii, TX, 1, NXI + p0 * TX + ii, TX, min(L::SY, TY + 1 - p0)};
   };
-  for (int e0 = tid; e0 < 4 * NI; e0 += NW * BT) {
-    T a[NW][6], b[NW][6], o[NW][4];
-    int at[NW];
-    bool ok[NW];
-#pragma unroll
-    for (int w = 0; w < NW; w++) {
-      const int e = min(e0 + w * BT, 4 * NI - 1);
-      const int m = e / NI, f = e % NI;
-      int base, ust, cdo, cst, cls, dir;
-      ok[w] = geo(f, base, ust, cdo, cst, cls, dir) && e0 + w * BT < 4 * NI;
-      at[w] = m * NI + f;
-      load_stencil(m, base, ust, cdo, cst, cls, dir, a[w], b[w]);
+  // cells past the tile (a strip shorter than the longest) read the last one
+  const T eps = (T)P.eps;
+  const bool js = weno_kind(P) == W_JS;
+  // flow variables: item = (field, variable, strip), field 0 u and 1 its flux
+  for (int e = tid; e < 8 * L::NSTR; e += BT) {
+    const int fv = e / L::NSTR, fld = fv >> 2, m = fv & 3;
+    const Strip w = strip(e - fv * L::NSTR);
+    const T* src;
+    int st;
+    if (fld == 0) {
+      if constexpr (MX) src = sUf + m * vs + w.u;
+      else src = sU + m * vs + w.u;
+      st = w.us;
+    } else {
+      if constexpr (MX) src = (w.dir ? cyf + m * NCY : cxf + m * NCX) + w.f;
+      else src = (w.dir ? cy + m * NCY : cx + m * NCX) + w.f;
+      st = w.fs;
     }
-    weno5_iface_n<NW, T>(P, a, b, o);
+    T* o = rec + (8 * fld + m) * NI + w.i;
+    const int last = w.n + 4;
+    if (js) {
+      weno5_strip_js<L::SMAX, 1, T>(
+          eps, [&](int, int k) { return src[min(k, last) * st]; },
+          [&](int r, const T* vL, const T* vR) {
+            if (r < w.n) { o[r * w.is] = vL[0]; o[r * w.is + 4 * NI] = vR[0]; }
+          });
+    } else {
+      for (int r = 0; r < w.n; r++) {
+        T c[6], vL, vR;
 #pragma unroll
-    for (int w = 0; w < NW; w++)
-      if (ok[w]) {
-        rec[at[w]] = o[w][0]; rec[at[w] + 4 * NI] = o[w][1]; rec[at[w] + 8 * NI] = o[w][2];
-        rec[at[w] + 12 * NI] = o[w][3];
+        for (int k = 0; k < 6; k++) c[k] = src[(r + k) * st];
+        weno5_pair(P, c, vL, vR);
+        o[r * w.is] = vL; o[r * w.is + 4 * NI] = vR;
       }
+    }
   }
   __syncthreads();
   for (int f = tid; f < NI; f += BT) {
-    int base, ust, cdo, cst, cls, dir;
-    if (!geo(f, base, ust, cdo, cst, cls, dir)) continue;
+    int base, ust, dir;
+    if (!geo(f, base, ust, dir)) continue;
     T* so = f < NXI ? fx + f : fy + (f - NXI);
-    iface_upwind_flow<NS2D, UPW, MX>(P, rec + f, 4 * NI, NI, sU + base - ust, sU + base, sU + c0, vs, dir, so,
+    upwind_by_scheme<NS2D, MX>(P, rec + f, 4 * NI, NI, sU + base - ust, sU + base, sU + c0, vs, dir, so,
                                      f < NXI ? NXI : NYI, spa + f, spm + f);
   }
   __syncthreads();
-  const int npi = (nv - 4) * NI;
-  for (int e0 = tid; e0 < npi; e0 += NW * BT) {
-    T a[NW][6], b[NW][6], o[NW][4];
-    int fi[NW], mi[NW];
-    bool ok[NW];
+  // passive variables: item = (variable, strip), u and its flux vn u together
+  for (int e = tid; e < (nv - 4) * L::NSTR; e += BT) {
+    const int m = 4 + e / L::NSTR;
+    const Strip w = strip(e - (m - 4) * L::NSTR);
+    T* o = w.dir ? fy + m * NYI + w.i - NXI : fx + m * NXI + w.i;
+    const int last = w.n + 4;
+    auto cell = [&](int n, int k, T u) -> T {   // n = 1: the flux at cell k, whose u is given
+      if constexpr (MX) return n == 0 ? u : (w.dir ? cyf + m * NCY : cxf + m * NCX)[w.f + k * w.fs];
+      else return n == 0 ? u : __dmul_rn((w.dir ? cy + 4 * NCY : cx + 4 * NCX)[w.f + k * w.fs], u);
+    };
+    auto ucell = [&](int k) -> T {
+      if constexpr (MX) return sUf[m * vs + w.u + k * w.us];
+      else return sU[m * vs + w.u + k * w.us];
+    };
+    auto put = [&](int r, const T* vL, const T* vR) {
+      const int f = w.i + r * w.is;
+      o[r * w.is] = upwind_species(spm[f], spa[f], vL[0], vR[0], vL[1], vR[1]);
+    };
+    if (js) {
+      weno5_strip_js<L::SMAX, 2, T>(
+          eps,
+          [&](int n, int k) {
+            const int kk = min(k, last);
+            return cell(n, kk, ucell(kk));
+          },
+          [&](int r, const T* vL, const T* vR) { if (r < w.n) put(r, vL, vR); });
+    } else {
+      for (int r = 0; r < w.n; r++) {
+        T c[2][6], vL[2], vR[2];
 #pragma unroll
-    for (int w = 0; w < NW; w++) {
-      const int e = min(e0 + w * BT, npi - 1);
-      const int m = 4 + e / NI, f = e % NI;
-      int base, ust, cdo, cst, cls, dir;
-      ok[w] = geo(f, base, ust, cdo, cst, cls, dir) && e0 + w * BT < npi;
-      fi[w] = f; mi[w] = m;
-      load_stencil(m, base, ust, cdo, cst, cls, dir, a[w], b[w]);
-    }
-    weno5_iface_n<NW, T>(P, a, b, o);
-#pragma unroll
-    for (int w = 0; w < NW; w++)
-      if (ok[w]) {
-        const int f = fi[w];
-        const T h = upwind_species(spm[f], spa[f], o[w][0], o[w][1], o[w][2], o[w][3]);
-        if (f < NXI) fx[mi[w] * NXI + f] = h;
-        else fy[mi[w] * NYI + f - NXI] = h;
+        for (int k = 0; k < 6; k++) { c[0][k] = ucell(r + k); c[1][k] = cell(1, r + k, c[0][k]); }
+        weno5_pair(P, c[0], vL[0], vR[0]);
+        weno5_pair(P, c[1], vL[1], vR[1]);
+        put(r, vL, vR);
       }
+    }
   }
   __syncthreads();
   // viscous fluxes (k_visc_source on this tile), in the work region; MX:
@@ -593,7 +645,7 @@ __device__ __forceinline__ void tile2d(const BMember& M, const BState& Sd, int s
   rk_point(M, Sd, s, p, nv);
 }
 
-template <int UPW, int BT, bool MX>
+template <int BT, bool MX>
 __device__ __forceinline__ void tile1d(const BMember& M, const BState& Sd, int s, int tx, char* smem) {
   typedef Tile1D<BT, MX> L;
   typedef typename L::T T;
@@ -624,7 +676,7 @@ __device__ __forceinline__ void tile1d(const BMember& M, const BState& Sd, int s
   __syncthreads();
   for (int f = tid; f < LX; f += BT) {
     if (i0 + f > N0) continue;
-    iface_upwind_flow<EULER1D, UPW, MX>(P, rec + f, NF * LX, LX, sU + f + H - 1, sU + f + H, sU + H, HX, 0, sF + f,
+    upwind_by_scheme<EULER1D, MX>(P, rec + f, NF * LX, LX, sU + f + H - 1, sU + f + H, sU + H, HX, 0, sF + f,
                                         LX, spa + f, spm + f);
   }
   __syncthreads();
@@ -668,19 +720,9 @@ __global__ void __launch_bounds__(BT, MINB) k_batch_stage(const BMember* __restr
     const int local = g - M.tile_off;
     if (M.P.ndims == 2) {
       const int tx = local % M.tnx, ty = local / M.tnx;
-      switch (M.P.upwind) {
-        case UPW_ROE: tile2d<TX, TY, UPW_ROE, BT, MX>(M, Sd, s, tx, ty, smem); break;
-        case UPW_RF: tile2d<TX, TY, UPW_RF, BT, MX>(M, Sd, s, tx, ty, smem); break;
-        case UPW_LLF: tile2d<TX, TY, UPW_LLF, BT, MX>(M, Sd, s, tx, ty, smem); break;
-        default: tile2d<TX, TY, UPW_RUSANOV, BT, MX>(M, Sd, s, tx, ty, smem); break;
-      }
+      tile2d<TX, TY, BT, MX>(M, Sd, s, tx, ty, smem);
     } else {
-      switch (M.P.upwind) {
-        case UPW_ROE: tile1d<UPW_ROE, BT, MX>(M, Sd, s, local, smem); break;
-        case UPW_RF: tile1d<UPW_RF, BT, MX>(M, Sd, s, local, smem); break;
-        case UPW_LLF: tile1d<UPW_LLF, BT, MX>(M, Sd, s, local, smem); break;
-        default: tile1d<UPW_RUSANOV, BT, MX>(M, Sd, s, local, smem); break;
-      }
+      tile1d<BT, MX>(M, Sd, s, local, smem);
     }
     __syncthreads();   // shared memory is reused by the next tile
   }

@@ -216,6 +216,43 @@ __device__ __forceinline__ T weno5_value(T w1, T w2, T w3, T m3, T m2, T m1, T p
   return w1 * f1 + w2 * f2 + w3 * f3;
 }
 
+// The pieces of WENO5 with the Jiang-Shu weights in its difference form.
+// weno5_js_window: from the two first differences g0, g1 of a window of three
+// cells, the squares of the smoothness indicators (at 4x, e4 = 4 eps) in which
+// the window is the far (q1), middle (q2) and near (q3) candidate of the
+// left-biased value.  weno5_js_offset: the value's offset from the cell beside
+// the interface, with weights a, 6 b, 3 e on the far, middle and near
+// candidates; d2, d1 the differences before that cell, dm the one across the
+// interface, dn the one after.  Every operation is rounded on its own or an
+// explicit fused one, so a value does not depend on the kernel or the loop that
+// forms it.
+template <typename T>
+__device__ __forceinline__ void weno5_js_window(T g0, T g1, T e4, T& q1, T& q2, T& q3) {
+  const T d = g1 - g0;
+  const T e1 = fma_rn(T(2), g1, d), e2 = g0 + g1, e3 = fma_rn(T(-2), g0, d);
+  const T dd = fma_rn(mul_rn(T(13.0 / 3.0), d), d, e4);
+  const T s1 = fma_rn(e1, e1, dd), s2 = fma_rn(e2, e2, dd), s3 = fma_rn(e3, e3, dd);
+  q1 = mul_rn(s1, s1); q2 = mul_rn(s2, s2); q3 = mul_rn(s3, s3);
+}
+template <typename T>
+__device__ __forceinline__ T weno5_js_offset(T a, T b, T e, T d2, T d1, T dm, T dn) {
+  const T f1 = fma_rn(T(5.0 / 6.0), d1, mul_rn(T(-1.0 / 3.0), d2));
+  const T f2 = fma_rn(T(2), dm, d1), f3 = fma_rn(T(2), dm, mul_rn(T(-0.5), dn));
+  const T den = fma_rn(T(6), b, fma_rn(T(3), e, a));
+  return mul_rn(fma_rn(a, f1, fma_rn(b, f2, mul_rn(e, f3))), rcp_nr(den));
+}
+// both biases at the interface of the cells c[0..5]
+template <typename T>
+__device__ __forceinline__ void weno5_js_pair(const T* c, T eps, T& vL, T& vR) {
+  T g[5], q1[4], q2[4], q3[4];
+#pragma unroll
+  for (int k = 0; k < 5; k++) g[k] = c[k + 1] - c[k];
+#pragma unroll
+  for (int t = 0; t < 4; t++) weno5_js_window(g[t], g[t + 1], T(4) * eps, q1[t], q2[t], q3[t]);
+  vL = c[2] + weno5_js_offset(mul_rn(q2[1], q3[2]), mul_rn(q1[0], q3[2]), mul_rn(q1[0], q2[1]), g[0], g[1], g[2], g[3]);
+  vR = c[3] - weno5_js_offset(mul_rn(q1[1], q2[2]), mul_rn(q1[1], q3[3]), mul_rn(q2[2], q3[3]), g[4], g[3], g[2], g[1]);
+}
+
 // The four WENO5 interface values at one interface (Interp1PrimFifthOrderWENO.c
 // for upw = +1 / -1 on u and f) with the weights of type WT (each value formed
 // from the unnormalised weights, then scaled by their normalisation): a[0..5] and
@@ -237,6 +274,12 @@ __device__ __forceinline__ void weno5_pair_t(const T* c, T eps, T& vL, T& vR) {
   if (WT == WT_NONE) {
     vL = weno5_value(c1, c2, c3, c[0], c[1], c[2], c[3], c[4]);
     vR = weno5_value(c1, c2, c3, c[5], c[4], c[3], c[2], c[1]);
+    return;
+  }
+  // FP64 Jiang-Shu in the difference form; the FP32 lines of mixed precision
+  // that come one interface at a time keep the six-cell form
+  if constexpr (WT == W_JS && sizeof(T) == 8) {
+    weno5_js_pair(c, eps, vL, vR);
     return;
   }
   const T t1343 = T(13.0 / 3.0);
@@ -269,6 +312,58 @@ template <int WT, typename T>
 __device__ __forceinline__ void weno5_iface_t(const T* a, const T* b, T eps, T& uL, T& uR, T& fL, T& fR) {
   weno5_pair_t<WT>(a, eps, uL, uR);
   weno5_pair_t<WT>(b, eps, fL, fR);
+}
+
+// WENO5 with the Jiang-Shu weights at S consecutive interfaces of NL lines at
+// once (the lines share nothing; their chains overlap): cell(n, k) is cell k
+// of line n, k = 0 .. S + 4, where interface r lies between cells r + 2 and
+// r + 3; put(r, vL, vR) takes the two biases of interface r of every line.
+//
+// Marching along a line shares what neighbouring interfaces have in common.
+// Per window of three cells, from the first differences g: the curvature and
+// slope terms of the three smoothness indicators (at 4x, eps folded in) and
+// their squares q.  The left weights of interface j and the right weights of
+// interface j - 1 are the same three products of q with the first and third
+// roles swapped.  Each candidate value is the cell beside the interface plus a
+// combination of two differences, so the value is that cell plus one quotient.
+// 46 FP64 operations an interface, line and pair of biases where the six-cell
+// form takes 92, and one cell read instead of six.
+template <int S, int NL, typename T, typename Cell, typename Put>
+__device__ __forceinline__ void weno5_strip_js(T eps, Cell cell, Put put) {
+  T c[NL][S + 5], g[NL][S + 4], q1[NL][S + 3], q2[NL][S + 3], q3[NL][S + 3];
+  T P23[NL][S + 1], P13[NL][S + 1], P12[NL][S + 1];
+  const T e4 = T(4) * eps;
+  auto next = [&](int n, int k) {   // cell k and the difference before it
+    c[n][k] = cell(n, k);
+    if (k > 0) g[n][k - 1] = c[n][k] - c[n][k - 1];
+  };
+  auto window = [&](int n, int t) { weno5_js_window(g[n][t], g[n][t + 1], e4, q1[n][t], q2[n][t], q3[n][t]); };
+  auto products = [&](int n, int j) {
+    P23[n][j] = mul_rn(q2[n][j + 1], q3[n][j + 2]);
+    P13[n][j] = mul_rn(q1[n][j], q3[n][j + 2]);
+    P12[n][j] = mul_rn(q1[n][j], q2[n][j + 1]);
+  };
+#pragma unroll
+  for (int n = 0; n < NL; n++) {
+#pragma unroll
+    for (int k = 0; k < 5; k++) next(n, k);
+    window(n, 0); window(n, 1); window(n, 2);
+    products(n, 0);
+  }
+#pragma unroll
+  for (int r = 0; r < S; r++) {
+    T vL[NL], vR[NL];
+#pragma unroll
+    for (int n = 0; n < NL; n++) {
+      next(n, r + 5);
+      window(n, r + 3);
+      products(n, r + 1);
+      const T* d = g[n] + r;
+      vL[n] = c[n][r + 2] + weno5_js_offset(P23[n][r], P13[n][r], P12[n][r], d[0], d[1], d[2], d[3]);
+      vR[n] = c[n][r + 3] - weno5_js_offset(P12[n][r + 1], P13[n][r + 1], P23[n][r + 1], d[4], d[3], d[2], d[1]);
+    }
+    put(r, vL, vR);
+  }
 }
 
 // the reconstruction of the explicit schemes: upw5, WENO5 with the optimal
