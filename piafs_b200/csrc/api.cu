@@ -106,52 +106,111 @@ void piafs::enqueue_recon(piafs_gpu_sim* s, const double* U, int d, double* cons
   mark();
 }
 
+// The reconstruction of both directions of a 2D grid: the y pass on its own
+// stream, concurrent with the x pass, where the simulation has one (and no
+// phase events are asked for); joined when this returns.
+static void enqueue_recon2d(piafs_gpu_sim* s, const double* U, cudaEvent_t* ev = nullptr, int* k = nullptr) {
+  const DevParams& P = s->P;
+  const bool concurrent = s->concurrent_y && !ev;
+  if (concurrent) cudaEventRecord(s->yfork, s->stream);
+  enqueue_recon(s, U, 0, s->iface, ev, k);
+  if (concurrent) {
+    // the y pass joins the x pass's stream before the kernel that ends the stage
+    cudaStreamWaitEvent(s->ystream, s->yfork, 0);
+    double* const* Iy = s->iface_y;
+    launch_transpose_flux_y(P, U, s->ut, s->fCy, s->ystream);
+    launch_crweno(s->PT, s->ut, s->fCy, Iy[0], Iy[1], Iy[2], Iy[3], 0, s->err, s->ystream);
+    cudaEventRecord(s->yjoin, s->ystream);
+    cudaStreamWaitEvent(s->stream, s->yjoin, 0);
+  } else {
+    enqueue_recon(s, U, 1, s->iface_y, ev, k);
+  }
+}
+
+// What ends a stage from the interface arrays of enqueue_recon2d: -hyp or hyp
+// alone into k, until the caller asks for more.
+static Stage2D stage2d_args(piafs_gpu_sim* s, const double* U, double* k, bool neg) {
+  Stage2D S{};
+  S.U = U;
+  S.UT = s->ut;
+  for (int i = 0; i < 4; i++) { S.xi[i] = s->iface[i]; S.yi[i] = s->iface_y[i]; }
+  S.dxinv = s->dxinv;
+  S.imap = s->imap;
+  S.neg = neg ? 1 : 0;
+  S.k = k;
+  return S;
+}
+
+// the fourth-order viscous terms have their own kernel, the source with them
+static bool visc4(const DevParams& P) { return P.viscous && P.par4; }
+
 // HyperbolicFunction (HyperbolicFunction.c:35-119) over all directions into
-// out: -hyp (neg, the stage derivative's first term) or hyp.  In 2D both
-// directions' interfaces are reconstructed first and one kernel upwinds them
-// and forms the divergence.
+// out: -hyp (neg, the stage derivative's first term) or hyp.
 static void enqueue_hyp(piafs_gpu_sim* s, const double* U, double* out, bool neg, cudaEvent_t* ev = nullptr,
                         int* k = nullptr) {
   const DevParams& P = s->P;
-  if (s->concurrent_y && !ev && P.ndims == 2) cudaEventRecord(s->yfork, s->stream);
-  enqueue_recon(s, U, 0, s->iface, ev, k);
   if (P.ndims == 1) {
+    enqueue_recon(s, U, 0, s->iface, ev, k);
     launch_upwind_div(P, U, s->iface[0], s->iface[1], s->iface[2], s->iface[3], s->dxinv, out, 0, neg ? 0 : 2,
                       s->stream);
   } else {
-    if (s->concurrent_y && !ev) {
-      // the y pass joins the x pass's stream before the upwind kernel
-      cudaStreamWaitEvent(s->ystream, s->yfork, 0);
-      double* const* Iy = s->iface_y;
-      launch_transpose_flux_y(P, U, s->ut, s->fCy, s->ystream);
-      launch_crweno(s->PT, s->ut, s->fCy, Iy[0], Iy[1], Iy[2], Iy[3], 0, s->err, s->ystream);
-      cudaEventRecord(s->yjoin, s->ystream);
-      cudaStreamWaitEvent(s->stream, s->yjoin, 0);
-    } else {
-      enqueue_recon(s, U, 1, s->iface_y, ev, k);
-    }
-    const void* xi[4] = {s->iface[0], s->iface[1], s->iface[2], s->iface[3]};
-    const void* yi[4] = {s->iface_y[0], s->iface_y[1], s->iface_y[2], s->iface_y[3]};
-    launch_upwind_div2d(P, U, s->ut, xi, yi, s->dxinv, out, neg ? 1 : 0, s->stream);
+    enqueue_recon2d(s, U, ev, k);
+    launch_stage2d(P, stage2d_args(s, U, out, neg), s->stream);
   }
   if (ev) cudaEventRecord(ev[++*k], s->stream);
 }
 
-// TimeRHSFunctionExplicit (TimeRHSFunctionExplicit.c:29-77) on SoA arrays:
-// rhs = -hyp + par + source; U must have its ghosts filled.
-// hnu: where the source stores the photon density of this evaluation (the
-// reference's Chemistry::nv_hnu), or nullptr
 // the sponge zones' source (SourceFunction.c:42-57) added to rhs
 static void enqueue_sponge(piafs_gpu_sim* s, const double* U, double* rhs) {
   for (const auto& z : s->sponges)
     launch_sponge(s->P, U, rhs, z.dim, z.is, z.ie, s->sponge_buf + z.sig_off, s->sponge_buf + z.ref_off, s->stream);
 }
 
+// The Runge-Kutta combination that follows a stage (TimeRK.c:60-75, :86-99):
+// dst = u + sum a[j] d[j] + as * (the stage's derivative).
+struct RkNext {
+  double* dst;
+  int nprev;
+  const double* d[MAX_STAGES];
+  double a[MAX_STAGES];
+  double as;
+};
+
+// TimeRHSFunctionExplicit (TimeRHSFunctionExplicit.c:29-77) on SoA arrays:
+// rhs = -hyp + par + source; U must have its ghosts filled.
+// hnu: where the source stores the photon density of this evaluation (the
+// reference's Chemistry::nv_hnu), or nullptr.  next (2D, s->fuse_rk): the
+// combination that follows, formed by the same kernel; keep: whether rhs is
+// read after it.
 static void enqueue_rhs(piafs_gpu_sim* s, double* rhs, const double* U, const double* tdev, double cstage,
-                        double* hnu = nullptr) {
-  enqueue_hyp(s, U, rhs, true);
-  launch_visc_source(s->P, U, s->dxinv, s->imap, tdev, cstage, rhs, 1, 1, s->stream, hnu);
+                        double* hnu = nullptr, const RkNext* next = nullptr, bool keep = true,
+                        cudaEvent_t* ev = nullptr, int* k = nullptr) {
+  const DevParams& P = s->P;
+  auto mark = [&]() { if (ev) cudaEventRecord(ev[++*k], s->stream); };
+  if (P.ndims == 1 || visc4(P)) {
+    enqueue_hyp(s, U, rhs, true, ev, k);
+    launch_visc_source(P, U, s->dxinv, s->imap, tdev, cstage, rhs, 1, 1, s->stream, hnu);
+  } else {
+    enqueue_recon2d(s, U, ev, k);
+    Stage2D S = stage2d_args(s, U, rhs, true);
+    S.visc = P.viscous;
+    S.chem = P.chem;
+    S.tdev = tdev;
+    S.cstage = cstage;
+    S.hnu = hnu;
+    if (next) {
+      S.dst = next->dst;
+      S.u = s->u;
+      S.nprev = next->nprev;
+      for (int j = 0; j < next->nprev; j++) { S.d[j] = next->d[j]; S.a[j] = next->a[j]; }
+      S.as = next->as;
+      if (!keep && !stage2d_stores_k(P, S.chem)) S.k = nullptr;
+    }
+    launch_stage2d(P, S, s->stream);
+    mark();
+  }
   enqueue_sponge(s, U, rhs);
+  mark();
 }
 
 void piafs::enqueue_bc(piafs_gpu_sim* s, double* u) {
@@ -160,29 +219,45 @@ void piafs::enqueue_bc(piafs_gpu_sim* s, double* u) {
 
 // One time step: TimePreStep's boundary conditions on u, TimeRK's stages and
 // step completion, t += dt.  U[0] aliases u: the reference copies u into
-// U[0] and re-applies the (idempotent) boundary conditions to it.
+// U[0] and re-applies the (idempotent) boundary conditions to it.  Where the
+// kernel that ends a stage forms the combination too, it writes the interior
+// points of the next stage's state (ghosts no zone writes keep u's values,
+// copied when the state was set); a step that asks for the norm completes
+// with the kernel that sums it.
 static void enqueue_step(piafs_gpu_sim* s, bool with_norm) {
   const DevParams& P = s->P;
   const Deck& d = s->deck;
   const int ns = d.nstages;
   const long long n = (long long)P.nvars * P.ps;
+  // coefficients of the state after stage st: the next stage's, or the step's
+  auto coef = [&](int st, int j) { return d.dt * (st < ns - 1 ? d.A[(st + 1) * MAX_STAGES + j] : d.b[j]); };
   enqueue_bc(s, s->u);
   for (int st = 0; st < ns; st++) {
     double* Us = st == 0 ? s->u : s->U[st];
-    if (st > 0) {
-      const double* dd[MAX_STAGES];
-      double a[MAX_STAGES];
-      for (int j = 0; j < st; j++) { dd[j] = s->Ud[j]; a[j] = d.dt * d.A[st * MAX_STAGES + j]; }
-      launch_stage(n, Us, s->u, dd, a, st, s->stream);
-      enqueue_bc(s, Us);
+    const bool last = st == ns - 1;
+    double* hnu = last ? s->hnu : nullptr;
+    if (s->fuse_rk && !(last && with_norm)) {
+      RkNext nx{};
+      nx.dst = last ? s->u : s->U[st + 1];
+      nx.nprev = st;
+      for (int j = 0; j < st; j++) { nx.d[j] = s->Ud[j]; nx.a[j] = coef(st, j); }
+      nx.as = coef(st, st);
+      enqueue_rhs(s, s->Ud[st], Us, s->tdev, d.c[st], hnu, &nx, !last);
+      if (!last) enqueue_bc(s, s->U[st + 1]);
+      continue;
     }
-    enqueue_rhs(s, s->Ud[st], Us, s->tdev, d.c[st], st == ns - 1 ? s->hnu : nullptr);
+    enqueue_rhs(s, s->Ud[st], Us, s->tdev, d.c[st], hnu);
+    const double* dd[MAX_STAGES];
+    double a[MAX_STAGES];
+    for (int j = 0; j <= st; j++) { dd[j] = s->Ud[j]; a[j] = coef(st, j); }
+    if (!last) {
+      launch_stage(n, s->U[st + 1], s->u, dd, a, st + 1, s->stream);
+      enqueue_bc(s, s->U[st + 1]);
+    } else {
+      if (with_norm) cudaMemsetAsync(s->norm_acc, 0, sizeof(double), s->stream);
+      launch_update(P, s->u, dd, a, ns, with_norm ? s->norm_acc : nullptr, s->stream);
+    }
   }
-  const double* dd[MAX_STAGES];
-  double b[MAX_STAGES];
-  for (int j = 0; j < ns; j++) { dd[j] = s->Ud[j]; b[j] = d.dt * d.b[j]; }
-  if (with_norm) cudaMemsetAsync(s->norm_acc, 0, sizeof(double), s->stream);
-  launch_update(P, s->u, dd, b, ns, with_norm ? s->norm_acc : nullptr, s->stream);
   launch_advance_time(s->tdev, d.dt, s->stream);
 }
 
@@ -254,13 +329,12 @@ int piafs::create_sim(Deck&& deck, int precision, piafs_gpu_sim** out) {
   s->precision = precision;
   s->P.mixed = precision == PIAFS_PRECISION_MIXED ? 1 : 0;
   {
-    // PIAFS_GPU_NO_PACKED_SPECIES=1 keeps the passive variables' four
-    // interface arrays (the same values; for checking the packed form)
+    // PIAFS_GPU_NO_PACKED_SPECIES=1 keeps the four interface arrays (the
+    // same values; for checking the packed form)
     const DevParams& Q = s->P;
     const char* npk = std::getenv("PIAFS_GPU_NO_PACKED_SPECIES");
-    s->P.pack_sp = (Q.model == NS2D && Q.ndims == 2 && Q.nvars > Q.nflow && Q.scheme == CRWENO5 &&
-                    !Q.char_interp && Q.upwind != UPW_RF && crweno_line_fits(Q.N0) && crweno_line_fits(Q.N1) &&
-                    !(npk && npk[0] == '1'))
+    s->P.pack_sp = (Q.model == NS2D && Q.ndims == 2 && !Q.char_interp && Q.upwind != UPW_RF &&
+                    (Q.scheme != CRWENO5 || (crweno_packs(Q.N0) && crweno_packs(Q.N1))) && !(npk && npk[0] == '1'))
                        ? 1 : 0;
   }
   if (s->P.mixed && s->P.char_interp) {
@@ -353,6 +427,9 @@ int piafs::create_sim(Deck&& deck, int precision, piafs_gpu_sim** out) {
     return fail(code, msg);
   }
   s->U[0] = s->u;
+  // one-stage schemes advance u itself, which other tiles still read as the
+  // stage's state: their combination stays a kernel of its own
+  s->fuse_rk = P.ndims == 2 && !visc4(P) && s->sponges.empty() && d.nstages > 1;
   // initial solution; restart time waqt = restart_iter * dt (TimeInitialize.c:51)
   int rr = piafs_gpu_set_state(s, d.u0.data(), d.restart_iter * d.dt);
   if (rr) { free_sim(s); return rr; }
@@ -391,13 +468,14 @@ int piafs_gpu_get_info(piafs_gpu_sim* s, piafs_gpu_info* info) {
   info->npoints_ghosted = s->P.npg;
   info->ninterfaces[0] = s->P.nint[0]; info->ninterfaces[1] = s->P.nint[1];
   info->cfl = s->last_cfl; info->norm = s->last_norm; info->singular = s->singular;
-  // kernels per step: the prestep BC launches (nz), per stage (combine + BCs for s > 0, flux
+  // kernels per step: the BC launches (nz) of every stage, per stage flux
   // and reconstruction per direction plus the transpose of a transposed y
-  // pass, one upwind/divergence kernel, viscous/source), update, clock
+  // pass and the upwind / stage kernel, the separate source and combination
+  // kernels where they are not part of it, and the clock
   const int nz = launch_bc(s->P, nullptr, d.zones.data(), (int)d.zones.size(), nullptr);
-  const int vs = ((s->P.ndims == 2 && s->P.viscous) || s->P.chem) ? 1 : 0;
+  const int vs = (((s->P.ndims == 2 && s->P.viscous) || s->P.chem) && (s->P.ndims == 1 || visc4(s->P))) ? 1 : 0;
   const int tr = (s->ut && s->P.model != NS2D) ? 1 : 0;   // NS2D: the transpose also forms the y flux
-  info->launches_per_step = nz + d.nstages * (2 * s->P.ndims + 1 + tr + vs) + (d.nstages - 1) * (1 + nz) + 2;
+  info->launches_per_step = d.nstages * (nz + 2 * s->P.ndims + 1 + tr + vs + (s->fuse_rk ? 0 : 1)) + 1;
   return PIAFS_OK;
 }
 
@@ -405,6 +483,7 @@ int piafs_gpu_set_state(piafs_gpu_sim* s, const double* u_host, double t) {
   if (!s || !u_host) return fail(PIAFS_ERR_ARGUMENT, "null argument");
   CK(cudaMemcpyAsync(s->aos, u_host, s->aos_bytes, cudaMemcpyHostToDevice, s->stream));
   launch_aos_to_soa(s->aos, s->u, s->P.npg, s->P.nvars, s->P.ps, s->stream);
+  if (s->fuse_rk) launch_copy_ghosts(s->P, s->u, s->U + 1, s->deck.nstages - 1, s->stream);
   CK(cudaMemcpyAsync(s->tdev, &t, sizeof(double), cudaMemcpyHostToDevice, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   s->t = t;
@@ -488,10 +567,7 @@ int piafs_gpu_profile_rhs(piafs_gpu_sim* s, int reps, double* ms, int* nphases) 
     enqueue_bc(s, U);
     int k = 0;
     CK(cudaEventRecord(ev[0], s->stream));
-    enqueue_hyp(s, U, R, true, ev.data(), &k);
-    launch_visc_source(P, U, s->dxinv, s->imap, s->tdev, 0.0, R, 1, 1, s->stream);
-    enqueue_sponge(s, U, R);
-    CK(cudaEventRecord(ev[++k], s->stream));
+    enqueue_rhs(s, R, U, s->tdev, 0.0, nullptr, nullptr, true, ev.data(), &k);
     CK(cudaStreamSynchronize(s->stream));
     if (r < 0) continue;
     for (int i = 0; i < np; i++) {
@@ -698,12 +774,10 @@ static int finish(piafs_gpu_sim* s) {
 
 int piafs_gpu_RHSFunction(piafs_gpu_sim* s, double* rhs, double* u, double t) {
   if (!s || !rhs || !u) return fail(PIAFS_ERR_ARGUMENT, "null argument");
-  const size_t planes = (size_t)s->P.nvars * s->P.ps * sizeof(double);
   double* U = s->scratch;
-  double* R = s->Ud[0];
+  double* R = s->Ud[0];   // its ghost entries are never written: zero
   to_soa(s, u, U);
   enqueue_bc(s, U);
-  CK(cudaMemsetAsync(R, 0, planes, s->stream));
   if (int r = set_top_t(s, t)) return r;
   enqueue_rhs(s, R, U, s->top_t, 0.0);
   launch_soa_to_aos(U, u, s->P.npg, s->P.nvars, s->P.ps, s->stream);
@@ -715,9 +789,8 @@ int piafs_gpu_HyperbolicFunction(piafs_gpu_sim* s, double* hyp, const double* u,
   if (!s || !hyp || !u) return fail(PIAFS_ERR_ARGUMENT, "null argument");
   const DevParams& P = s->P;
   double* U = s->scratch;
-  double* H = s->Ud[0];
+  double* H = s->Ud[0];   // its ghost entries are never written: zero
   to_soa(s, u, U);
-  CK(cudaMemsetAsync(H, 0, (size_t)P.nvars * P.ps * sizeof(double), s->stream));
   enqueue_hyp(s, U, H, false);
   launch_soa_to_aos(H, hyp, P.npg, P.nvars, P.ps, s->stream);
   return finish(s);

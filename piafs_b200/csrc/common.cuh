@@ -52,12 +52,18 @@ struct DevParams {
   // rows [jg0, jg0 + N1) of a grid of N1g rows (a row slab of a decomposed
   // grid); 0 and N1 for a whole grid
   int jg0, N1g;
-  // 1: the CRWENO5 line solve stores the passive variables' interface values
-  // packed for their scalar upwinding -- uL - uR in the uL array, fL + fR in
-  // the fL array -- and the upwind kernels read them so (2D Navier-Stokes,
-  // upwinding other than RF)
+  // 1: the component reconstruction stores what the upwinding needs of the
+  // two biases (2D Navier-Stokes, upwinding other than RF): fL + fR in the fL
+  // array, and uL - uR in the uL array for the passive variables and, with
+  // Roe and Rusanov, the flow variables (LLF averages the interface states
+  // themselves); the kernels that read them do so accordingly
   int pack_sp;
 };
+
+// whether the reconstruction of variable v (of the flux, or of u) is packed
+__host__ __device__ inline bool packs(const DevParams& P, int v, bool flux) {
+  return P.pack_sp && (flux || v >= P.nflow || P.upwind != UPW_LLF);
+}
 
 __host__ __device__ inline long long pidx(const DevParams& P, int i, int j) {
   return (long long)(i + P.ghosts) + (long long)P.W0 * (long long)(j + P.g1);

@@ -77,14 +77,14 @@ __global__ void __launch_bounds__(line_threads_max(), 1)
   int bad = 0;
   line_pair_solve<M, WT, R, O>(P, src, st, ref, N, cs, pcA, tp, sy, so, bad);
   if (bad) atomicOr(err, 1);
-  // N + 1 interfaces over Pt threads: at most M + 1 each; the passive
-  // variables packed for their upwinding when P.pack_sp (uL - uR, fL + fR)
+  // N + 1 interfaces over Pt threads: at most M + 1 each; packed for the
+  // upwinding where it takes them so (uL - uR, fL + fR)
   const O* o = so + padm<M>(k);
   const int ostride = padm<M>(N) + 1, ostep = Pt + Pt / M;   // Pt is a multiple of M
   oL += k * ist;
   oR += k * ist;
   const long long gstep = Pt * ist;
-  if (P.pack_sp && v >= P.nflow) {
+  if (packs(P, v, isF)) {
 #pragma unroll
     for (int it = 0; it <= M; it++) {
       if (k + it * Pt <= N) {
@@ -298,6 +298,13 @@ __global__ void __launch_bounds__(line_threads_max(), 1)
   __syncthreads();
   const int lo = rank == 0 ? 0 : rb + 1;
   const int hi = kN / Pt == rank ? N : min(N - 1, rb + Pt * M);
+  if (packs(P, v, isF)) {
+    for (int i = lo + k; i <= hi; i += Pt) {
+      const O l = so[padm<M>(i - rb)], r = so[ostride + padm<M>(i - rb)];
+      oL[i * ist] = isF ? l + r : l - r;
+    }
+    return;
+  }
   for (int i = lo + k; i <= hi; i += Pt) {
     oL[i * ist] = so[padm<M>(i - rb)];
     oR[i * ist] = so[ostride + padm<M>(i - rb)];
@@ -395,6 +402,8 @@ void line_launch_m(const DevParams& P, const double* U, const double* F, void* u
 // lines of 3 .. 4097 interfaces: 8 rows per thread from 128 interfaces up
 // (up to 512 threads), 4 below
 bool crweno_line_fits(int N) { return N >= 3 && line_threads_m<8>(N) <= line_threads_max(); }
+
+bool crweno_packs(int N) { return crweno_line_fits(N) || crweno_cluster_size(N) > 1; }
 
 // lines of 4098 .. 32769 interfaces: clusters of up to 8 CTAs
 int launch_crweno_seg(const DevParams& P, const double* U, const double* F, void* uL, void* uR, void* fL, void* fR,

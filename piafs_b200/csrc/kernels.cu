@@ -7,11 +7,11 @@
 //   k_weno5 or      interface values uL,uR,fL,fR (InterpolateInterfacesHyp
 //   k_crw_line        with the weights of SetInterpLimiterVar fused in;
 //                     crweno_line.cu, crweno.cu)
-//   k_upwind_div2d  upwind flux at the interfaces of both directions +
-//   (k_upwind_div   conservative difference into the stage derivative
-//    in 1D)         (Upwind + HyperbolicFunction's dxinv*(fI[j+1]-fI[j]))
-// then k_visc_source (ParabolicFunction + SourceFunction) and the RK
-// kernels k_stage / k_update2 (TimeRK).  All state is FP64.
+// then in 2D k_stage2d (stage2d.cu: upwinding, divergence, viscous terms,
+// source and the Runge-Kutta combination), in 1D k_upwind_div (upwind flux and
+// conservative difference into the stage derivative, Upwind +
+// HyperbolicFunction's dxinv*(fI[j+1]-fI[j])) and the RK kernels k_stage /
+// k_update2 (TimeRK).  All state is FP64.
 #include <algorithm>
 #include <cstdio>
 #include <type_traits>
@@ -164,6 +164,32 @@ __global__ void __launch_bounds__(256) k_transpose_flux_y(DevParams P, const dou
       }
     }
   }
+}
+
+// The ghost points of a state copied to others: entry v of a ghost that no
+// boundary zone writes (corners; the passive variables at walls) keeps its
+// value through a step, in the stage states too.
+struct GhostDst {
+  double* p[MAX_STAGES];
+};
+__global__ void k_copy_ghosts(DevParams P, const double* __restrict__ u, GhostDst dst, int n) {
+  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int v = blockIdx.y, g = P.ghosts, g1 = P.g1;
+  const long long edge = 2LL * g1 * P.W0, side = 2LL * g * P.N1;   // whole rows below and above; the sides
+  if (e >= edge + side) return;
+  int i, j;
+  if (e < edge) {
+    i = (int)(e % P.W0) - g;
+    j = (int)(e / P.W0);
+    j = j < g1 ? j - g1 : P.N1 + j - g1;
+  } else {
+    const int k = (int)((e - edge) % (2 * g));
+    i = k < g ? k - g : P.N0 + k - g;
+    j = (int)((e - edge) / (2 * g));
+  }
+  const long long p = v * P.ps + pidx(P, i, j);
+  const double x = u[p];
+  for (int q = 0; q < n; q++) dst.p[q][p] = x;
 }
 
 // ================================================================ boundaries
@@ -382,7 +408,12 @@ __global__ void k_weno5(DevParams P, const double* __restrict__ U, const double*
   for (int r = 0; r < 6; r++) { a[r] = (R)(u[(r - 3) * st] - ru); b[r] = (R)(f[(r - 3) * st] - rf); }
   const long long o = (long long)v * P.pis + q;
   R* uL = (R*)uLv; R* uR = (R*)uRv; R* fL = (R*)fLv; R* fR = (R*)fRv;
-  weno5_iface(P, a, b, uL[o], uR[o], fL[o], fR[o]);
+  R w[4];
+  weno5_iface(P, a, b, w[0], w[1], w[2], w[3]);
+  if (packs(P, v, false)) uL[o] = w[0] - w[1];
+  else { uL[o] = w[0]; uR[o] = w[1]; }
+  if (packs(P, v, true)) fL[o] = w[2] + w[3];
+  else { fL[o] = w[2]; fR[o] = w[3]; }
 }
 
 // ======================================================== WENO5 (characteristic)
@@ -533,214 +564,6 @@ __global__ void __launch_bounds__(256) k_upwind_div(DevParams P, const double* _
     else if (mode == 2) *r = h;
     else *r = *r + h;
   }
-}
-
-// Upwind flux of all components at one interface q of direction DIR into
-// so[m * sm_stride] (NavierStokes2DUpwind*); cells pL / pR are the cells left
-// and right of the interface in `cells`.  MX: the interface arrays hold
-// floats relative to the line's reference values, uref (absolute, FP64) are
-// those references for the flow variables, the flux is computed in FP32 in
-// deviation form and stored relative to the line's flux reference.
-template <int UPW, int DIR, bool MX>
-__device__ __forceinline__ void iface_upwind(const DevParams& P, const void* __restrict__ uLv,
-                                             const void* __restrict__ uRv, const void* __restrict__ fLv,
-                                             const void* __restrict__ fRv, long long q,
-                                             const double* __restrict__ cells, long long pL, long long pR,
-                                             const double* uref,
-                                             typename std::conditional<MX, float, double>::type* so, int sm_stride) {
-  typedef typename std::conditional<MX, float, double>::type T;
-  constexpr int NF = Flow<NS2D>::NF;
-  const T* uL = (const T*)uLv; const T* uR = (const T*)uRv;
-  const T* fL = (const T*)fLv; const T* fR = (const T*)fRv;
-  T a[4], b[4], c[4], d[4], ucl[4], ucr[4], fi[4], spa;
-  int spm;
-#pragma unroll
-  for (int m = 0; m < NF; m++) {
-    a[m] = uL[m * P.pis + q]; b[m] = uR[m * P.pis + q];
-    c[m] = fL[m * P.pis + q]; d[m] = fR[m * P.pis + q];
-    if (UPW != UPW_LLF) { ucl[m] = (T)cells[m * P.ps + pL]; ucr[m] = (T)cells[m * P.ps + pR]; }
-  }
-  if (MX) {
-    T aL[4], aR[4];
-    if (UPW == UPW_LLF || UPW == UPW_RF) {
-#pragma unroll
-      for (int m = 0; m < NF; m++) { const T r = (T)uref[m]; aL[m] = r + a[m]; aR[m] = r + b[m]; }
-    }
-    upwind_flow_dev<NS2D, UPW, T>(a, b, c, d, aL, aR, ucl, ucr, (T)P.gamma, DIR, fi, &spa, &spm);
-  } else {
-    upwind_flow<NS2D, UPW, T>(a, b, c, d, ucl, ucr, (T)P.gamma, DIR, fi, &spa, &spm);
-  }
-#pragma unroll
-  for (int m = 0; m < NF; m++) so[m * sm_stride] = fi[m];
-  if (P.pack_sp) {
-    // passive variables packed by the line solve: uL - uR, fL + fR
-    int m = NF;
-    for (; m + 4 <= P.nvars; m += 4) {
-      T du[4], sf[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const long long o = (long long)(m + k) * P.pis + q;
-        du[k] = uL[o]; sf[k] = fL[o];
-      }
-#pragma unroll
-      for (int k = 0; k < 4; k++) so[(m + k) * sm_stride] = upwind_species_packed(spm, spa, du[k], sf[k]);
-    }
-    for (; m < P.nvars; m++)
-      so[m * sm_stride] = upwind_species_packed(spm, spa, uL[m * P.pis + q], fL[m * P.pis + q]);
-    return;
-  }
-  // passive variables four at a time, their sixteen loads in flight together
-  int m = NF;
-  for (; m + 4 <= P.nvars; m += 4) {
-    T l[4], r[4], fl[4], fr[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const long long o = (long long)(m + k) * P.pis + q;
-      l[k] = uL[o]; r[k] = uR[o]; fl[k] = fL[o]; fr[k] = fR[o];
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++) so[(m + k) * sm_stride] = upwind_species(spm, spa, l[k], r[k], fl[k], fr[k]);
-  }
-  for (; m < P.nvars; m++)
-    so[m * sm_stride] = upwind_species(spm, spa, uL[m * P.pis + q], uR[m * P.pis + q], fL[m * P.pis + q],
-                                       fR[m * P.pis + q]);
-}
-
-// Both directions of the 2D hyperbolic term in one pass: upwind fluxes at the
-// x and y interfaces of a 16 x 15 tile (one of each per thread), then
-// hyp = dxinv_x (fIx[i+1] - fIx[i]) + dxinv_y (fIy[j+1] - fIy[j])
-// (HyperbolicFunction.c:97-112, the x term first) and rhs = -hyp (neg = 1,
-// TimeRHSFunctionExplicit.c:64-66) or out = hyp (neg = 0): the same sum, in
-// the same order, that the per-direction kernels accumulate, with the stage
-// derivative written once.  The y-interface arrays are in the transposed
-// layout (q = j + (N1+1) i, cell values from UT) when YT, else in the
-// standard one (q = i + N0 j, cell values from U).  MX: mixed precision (FP32
-// interface values relative to their line's reference, FP32 fluxes and
-// differences, FP64 result).
-template <int UPW, bool YT, bool MX, bool HYIN>
-__global__ void __launch_bounds__(256, 3) k_upwind_div2d(DevParams P, const double* __restrict__ U,
-                                                      const double* __restrict__ UT,
-                                                      const void* __restrict__ xuL, const void* __restrict__ xuR,
-                                                      const void* __restrict__ xfL, const void* __restrict__ xfR,
-                                                      const void* __restrict__ yuL, const void* __restrict__ yuR,
-                                                      const void* __restrict__ yfL, const void* __restrict__ yfR,
-                                                      const double* __restrict__ dxinv, double* __restrict__ rhs,
-                                                      int neg, const void* __restrict__ hyin, int n0) {
-  typedef typename std::conditional<MX, float, double>::type T;
-  extern __shared__ double sfd[];
-  T* sf = (T*)sfd;
-  constexpr int TI = 16, TJ = 15, LX = TI + 1, LY = TJ + 2;   // LY padded against bank conflicts
-  constexpr int NX = LX * TJ, NY = TI * LY;
-  const int nvars = P.nvars, N0 = P.N0, N1 = P.N1, g = P.ghosts;
-  const int i0 = blockIdx.x * TI, j0 = blockIdx.y * TJ;
-  const int tid = threadIdx.x;
-  T* sx = sf;               // x-interface fluxes [m][row jj][ii = 0..TI]
-  T* sy = sf + nvars * NX;  // y-interface fluxes [m][column ii][jj = 0..TJ]
-  double uref[4];
-  if (tid < NX) {                // (TI + 1) x TJ x-interfaces
-    const int ii = tid % LX, jj = tid / LX;
-    const int i = i0 + ii, j = j0 + jj;
-    if (i <= N0 && j < N1) {
-      const long long pR = pidx(P, i, j);
-      if (MX && (UPW == UPW_LLF || UPW == UPW_RF)) {
-        const long long p0 = pidx(P, 0, j);
-#pragma unroll
-        for (int m = 0; m < 4; m++) uref[m] = U[m * P.ps + p0];
-      }
-      iface_upwind<UPW, 0, MX>(P, xuL, xuR, xfL, xfR, i + (long long)(N0 + 1) * j, U, pR - 1, pR, uref,
-                               sx + jj * LX + ii, NX);
-    }
-  }
-  if (!HYIN) {                   // TI x (TJ + 1) y-interfaces
-    int ii, jj;
-    if (YT) { jj = tid % (TJ + 1); ii = tid / (TJ + 1); }
-    else { ii = tid % TI; jj = tid / TI; }
-    const int i = i0 + ii, j = j0 + jj;
-    if (j <= N1 && i < N0) {
-      if (MX && (UPW == UPW_LLF || UPW == UPW_RF)) {
-        const long long p0 = pidx(P, i, 0);
-#pragma unroll
-        for (int m = 0; m < 4; m++) uref[m] = U[m * P.ps + p0];
-      }
-      if (YT) {
-        const long long pR = (long long)(j + g) + (long long)P.W1 * (i + g);
-        iface_upwind<UPW, 1, MX>(P, yuL, yuR, yfL, yfR, j + (long long)(N1 + 1) * i, UT, pR - 1, pR, uref,
-                                 sy + ii * LY + jj, NY);
-      } else {
-        const long long pR = pidx(P, i, j);
-        iface_upwind<UPW, 1, MX>(P, yuL, yuR, yfL, yfR, i + (long long)N0 * j, U, pR - P.W0, pR, uref,
-                                 sy + ii * LY + jj, NY);
-      }
-    }
-  }
-  __syncthreads();
-  if (tid >= TI * TJ) return;
-  const int ii = tid % TI, jj = tid / TI;
-  const int i = i0 + ii, j = j0 + jj;
-  if (i >= N0 || j >= N1) return;
-  const long long p = pidx(P, i, j);
-  const T dxi = (T)dxinv[g + i], dyi = (T)dxinv[P.W0 + g + j];
-  // HYIN: the y term of column i comes from the slab that owns it, as
-  // hyin[((i / n0) nvars + m) N1 + j) n0 + i % n0] (k_slab_upwind_y)
-  const T* hyv = (const T*)hyin;
-  const long long hbase = HYIN ? (long long)(i / n0) * nvars * N1 * n0 + (long long)j * n0 + i % n0 : 0;
-  for (int m = 0; m < nvars; m++) {
-    // hyp = dxinv_x dfx + dxinv_y dfy as dxinv_x dfx fused onto the rounded y
-    // term, on both paths
-    const T dfx = sx[m * NX + jj * LX + ii + 1] - sx[m * NX + jj * LX + ii];
-    const T hy = HYIN ? hyv[hbase + (long long)m * N1 * n0]
-                      : mul_rn(dyi, sy[m * NY + ii * LY + jj + 1] - sy[m * NY + ii * LY + jj]);
-    const double h = (double)fma_rn(dxi, dfx, hy);
-    rhs[(long long)m * P.ps + p] = neg ? -h : h;
-  }
-}
-
-// The y term of the 2D hyperbolic divergence on a column slab of a grid
-// decomposed along y (columns [c0, c0 + N0) of the whole grid, all N1 rows,
-// in the transposed layout: cell values from UT, interface q = j + (N1 + 1) c):
-// the upwind fluxes at the y interfaces of a 16 x 15 tile as in
-// k_upwind_div2d, then dyinv_j (fIy[j+1] - fIy[j]) for every variable,
-// written for the row slab that owns row j: hy[((r nvars + m) n1 + j - r n1)
-// N0 + c], r = j / n1.  The product is rounded on its own; k_upwind_div2d
-// fuses the x term's product onto it.
-template <int UPW, bool MX>
-__global__ void __launch_bounds__(256, 3) k_slab_upwind_y(DevParams P, const double* __restrict__ UT,
-                                                       const void* __restrict__ yuL, const void* __restrict__ yuR,
-                                                       const void* __restrict__ yfL, const void* __restrict__ yfR,
-                                                       const double* __restrict__ dyinv, void* __restrict__ hy,
-                                                       int n1) {
-  typedef typename std::conditional<MX, float, double>::type T;
-  extern __shared__ double sfd[];
-  T* sy = (T*)sfd;
-  constexpr int TI = 16, TJ = 15, LY = TJ + 2, NY = TI * LY;
-  const int nvars = P.nvars, N0 = P.N0, N1 = P.N1, g = P.ghosts;
-  const int i0 = blockIdx.x * TI, j0 = blockIdx.y * TJ;
-  const int tid = threadIdx.x;
-  double uref[4];
-  {
-    const int jj = tid % (TJ + 1), ii = tid / (TJ + 1);
-    const int i = i0 + ii, j = j0 + jj;
-    if (ii < TI && j <= N1 && i < N0) {
-      const long long line = (long long)P.W1 * (i + g);
-      if (MX && (UPW == UPW_LLF || UPW == UPW_RF)) {
-#pragma unroll
-        for (int m = 0; m < 4; m++) uref[m] = UT[m * P.ps + g + line];
-      }
-      const long long pR = (long long)(j + g) + line;
-      iface_upwind<UPW, 1, MX>(P, yuL, yuR, yfL, yfR, j + (long long)(N1 + 1) * i, UT, pR - 1, pR, uref,
-                               sy + ii * LY + jj, NY);
-    }
-  }
-  __syncthreads();
-  if (tid >= TI * TJ) return;
-  const int ii = tid % TI, jj = tid / TI;
-  const int i = i0 + ii, j = j0 + jj;
-  if (i >= N0 || j >= N1) return;
-  const T dyi = (T)dyinv[g + j];
-  const int r = j / n1;
-  T* out = (T*)hy + ((long long)r * nvars * n1 + (j - (long long)r * n1)) * N0 + i;
-  for (int m = 0; m < nvars; m++)
-    out[(long long)m * n1 * N0] = mul_rn(dyi, sy[m * NY + ii * LY + jj + 1] - sy[m * NY + ii * LY + jj]);
 }
 
 // ===================================================== viscous + chemistry
@@ -1163,6 +986,12 @@ int launch_bc(const DevParams& P, double* u, const Zone* z, int nz, cudaStream_t
   }
   return launches;
 }
+void launch_copy_ghosts(const DevParams& P, const double* u, double* const* dst, int n, cudaStream_t s) {
+  GhostDst D{};
+  for (int k = 0; k < n; k++) D.p[k] = dst[k];
+  const long long ghosts = 2LL * P.g1 * P.W0 + 2LL * P.ghosts * P.N1;
+  if (n > 0 && ghosts > 0) k_copy_ghosts<<<dim3(nblk(ghosts, 128), P.nvars), 128, 0, s>>>(P, u, D, n);
+}
 void launch_stage(long long n, double* Us, const double* u, const double* const* d, const double* a, int nterms,
                   cudaStream_t s) {
   k_stage<<<nblk(n, 256), 256, 0, s>>>(n, Us, u, nterms > 0 ? d[0] : nullptr, nterms > 0 ? a[0] : 0.0,
@@ -1268,70 +1097,6 @@ void launch_upwind_div(const DevParams& P, const double* U, const void* uL, cons
                        const void* fR, const double* dxinv, double* rhs, int dir, int mode, cudaStream_t s) {
   if (P.model == NS2D) upwind_div_model<NS2D>(P, U, uL, uR, fL, fR, dxinv, rhs, dir, mode, s);
   else upwind_div_model<EULER1D>(P, U, uL, uR, fL, fR, dxinv, rhs, dir, mode, s);
-}
-
-template <int UPW, bool YT, bool MX, bool HYIN>
-static void upwind_div2d_u(const DevParams& P, const double* U, const double* UT, const void* const* xi,
-                           const void* const* yi, const double* dxinv, double* rhs, int neg, const void* hyin,
-                           int n0, cudaStream_t s) {
-  raise_smem_limit<k_upwind_div2d<UPW, YT, MX, HYIN>>(200 * 1024);
-  dim3 grid(nblk(P.N0, 16), nblk(P.N1, 15));
-  size_t smem = (size_t)P.nvars * (17 * 15 + (HYIN ? 0 : 16 * 17)) * (MX ? sizeof(float) : sizeof(double));
-  const void* none = nullptr;
-  k_upwind_div2d<UPW, YT, MX, HYIN><<<grid, 256, smem, s>>>(P, U, UT, xi[0], xi[1], xi[2], xi[3],
-                                                             HYIN ? none : yi[0], HYIN ? none : yi[1],
-                                                             HYIN ? none : yi[2], HYIN ? none : yi[3], dxinv, rhs,
-                                                             neg, hyin, n0);
-}
-template <bool YT, bool MX, bool HYIN>
-static void upwind_div2d_yt(const DevParams& P, const double* U, const double* UT, const void* const* xi,
-                            const void* const* yi, const double* dxinv, double* rhs, int neg, const void* hyin,
-                            int n0, cudaStream_t s) {
-  switch (P.upwind) {
-    case UPW_ROE: upwind_div2d_u<UPW_ROE, YT, MX, HYIN>(P, U, UT, xi, yi, dxinv, rhs, neg, hyin, n0, s); break;
-    case UPW_RF: upwind_div2d_u<UPW_RF, YT, MX, HYIN>(P, U, UT, xi, yi, dxinv, rhs, neg, hyin, n0, s); break;
-    case UPW_RUSANOV: upwind_div2d_u<UPW_RUSANOV, YT, MX, HYIN>(P, U, UT, xi, yi, dxinv, rhs, neg, hyin, n0, s); break;
-    default: upwind_div2d_u<UPW_LLF, YT, MX, HYIN>(P, U, UT, xi, yi, dxinv, rhs, neg, hyin, n0, s); break;
-  }
-}
-void launch_upwind_div2d(const DevParams& P, const double* U, const double* UT, const void* const* xi,
-                         const void* const* yi, const double* dxinv, double* rhs, int neg, cudaStream_t s) {
-  if (P.mixed) {
-    if (UT) upwind_div2d_yt<true, true, false>(P, U, UT, xi, yi, dxinv, rhs, neg, nullptr, 0, s);
-    else upwind_div2d_yt<false, true, false>(P, U, UT, xi, yi, dxinv, rhs, neg, nullptr, 0, s);
-  } else {
-    if (UT) upwind_div2d_yt<true, false, false>(P, U, UT, xi, yi, dxinv, rhs, neg, nullptr, 0, s);
-    else upwind_div2d_yt<false, false, false>(P, U, UT, xi, yi, dxinv, rhs, neg, nullptr, 0, s);
-  }
-}
-void launch_upwind_div2d_hy(const DevParams& P, const double* U, const void* const* xi, const double* dxinv,
-                            const void* hy, int n0, double* rhs, int neg, cudaStream_t s) {
-  const void* const* none = xi;   // y interface arrays are not read
-  if (P.mixed) upwind_div2d_yt<false, true, true>(P, U, nullptr, xi, none, dxinv, rhs, neg, hy, n0, s);
-  else upwind_div2d_yt<false, false, true>(P, U, nullptr, xi, none, dxinv, rhs, neg, hy, n0, s);
-}
-template <int UPW, bool MX>
-static void slab_upwind_y_u(const DevParams& P, const double* UT, const void* const* yi, const double* dyinv,
-                            void* hy, int n1, cudaStream_t s) {
-  raise_smem_limit<k_slab_upwind_y<UPW, MX>>(200 * 1024);
-  dim3 grid(nblk(P.N0, 16), nblk(P.N1, 15));
-  size_t smem = (size_t)P.nvars * (16 * 17) * (MX ? sizeof(float) : sizeof(double));
-  k_slab_upwind_y<UPW, MX><<<grid, 256, smem, s>>>(P, UT, yi[0], yi[1], yi[2], yi[3], dyinv, hy, n1);
-}
-template <bool MX>
-static void slab_upwind_y_m(const DevParams& P, const double* UT, const void* const* yi, const double* dyinv,
-                            void* hy, int n1, cudaStream_t s) {
-  switch (P.upwind) {
-    case UPW_ROE: slab_upwind_y_u<UPW_ROE, MX>(P, UT, yi, dyinv, hy, n1, s); break;
-    case UPW_RF: slab_upwind_y_u<UPW_RF, MX>(P, UT, yi, dyinv, hy, n1, s); break;
-    case UPW_RUSANOV: slab_upwind_y_u<UPW_RUSANOV, MX>(P, UT, yi, dyinv, hy, n1, s); break;
-    default: slab_upwind_y_u<UPW_LLF, MX>(P, UT, yi, dyinv, hy, n1, s); break;
-  }
-}
-void launch_slab_upwind_y(const DevParams& P, const double* UT, const void* const* yi, const double* dyinv, void* hy,
-                          int n1, cudaStream_t s) {
-  if (P.mixed) slab_upwind_y_m<true>(P, UT, yi, dyinv, hy, n1, s);
-  else slab_upwind_y_m<false>(P, UT, yi, dyinv, hy, n1, s);
 }
 
 void launch_visc_source(const DevParams& P, const double* U, const double* dxinv, const double* imap,

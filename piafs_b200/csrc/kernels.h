@@ -184,6 +184,9 @@ int launch_crweno(const DevParams& P, const double* U, const double* F, void* uL
 // (crweno_line.cu): true if it serves lines of N points; -1 from the
 // launcher otherwise
 bool crweno_line_fits(int N);
+// whether lines of N points can store packed interface values (all but those
+// of fewer than three interfaces)
+bool crweno_packs(int N);
 int launch_crweno_line(const DevParams& P, const double* U, const double* F, void* uL, void* uR, void* fL,
                        void* fR, int dir, int* err, cudaStream_t s);
 // longer lines (up to 32769 interfaces) by clusters of CTAs that solve their
@@ -200,18 +203,45 @@ void launch_crweno_char(const DevParams& P, const double* U, const double* F, do
                         double* fR, int dir, double* scratch, int* err, cudaStream_t s);
 // mode 0: rhs = -hyp_x; 1: rhs = -((-rhs) + hyp_y); 2: out = hyp_x; 3: out += hyp_y
 // (interface arrays as written by launch_weno5 / launch_crweno; the mixed
-// variant covers the 1D x direction, 2D goes through launch_upwind_div2d)
+// variant covers the 1D x direction, 2D goes through launch_stage2d)
 void launch_upwind_div(const DevParams& P, const double* U, const void* uL, const void* uR, const void* fL,
                        const void* fR, const double* dxinv, double* rhs, int dir, int mode, cudaStream_t s);
-// both directions of a 2D hyperbolic term in one pass: xi / yi are the
-// (uL, uR, fL, fR) interface arrays of x and y; y in the transposed layout
-// with cell values from UT when UT is given.  rhs = -hyp (neg) or hyp.
-void launch_upwind_div2d(const DevParams& P, const double* U, const double* UT, const void* const* xi,
-                         const void* const* yi, const double* dxinv, double* rhs, int neg, cudaStream_t s);
-// the same with the y term given: hy from the column slabs of a grid
-// decomposed along y (launch_slab_upwind_y's layout, n0 columns per slab)
-void launch_upwind_div2d_hy(const DevParams& P, const double* U, const void* const* xi, const double* dxinv,
-                            const void* hy, int n0, double* rhs, int neg, cudaStream_t s);
+// What ends a 2D Runge-Kutta stage after the reconstruction (stage2d.cu): from
+// the (uL, uR, fL, fR) interface arrays of x and y (y in the transposed layout
+// with cell values from UT when UT is given) the hyperbolic term; or with the
+// y term given, from the column slabs of a grid decomposed along y
+// (launch_slab_upwind_y's layout, n0 columns per slab).  Then, as selected,
+// the viscous terms (second-order) and the photochemical source, and the
+// Runge-Kutta combination dst = u + sum_q a[q] d[q] + as k.
+struct Stage2D {
+  const double* U;               // the stage's state, ghosts filled
+  const double* UT;
+  const void* xi[4];
+  const void* yi[4];
+  const void* hy;
+  int n0;
+  const double* dxinv;
+  const double* imap;
+  const double* tdev;
+  double cstage;
+  int neg;                       // 1: k = -hyp + ...; 0: k = hyp
+  int visc, chem;
+  double* hnu;                   // photon density planes [nz][ps], or null
+  double* k;                     // the stage derivative (null: not stored; see stage2d_stores_k)
+  double* dst;                   // the combination, or null; not U
+  const double* u;
+  int nprev;
+  const double* d[MAX_STAGES];
+  double a[MAX_STAGES];
+  double as;
+};
+// whether k must be given (its kernel forms the derivative through memory)
+inline bool stage2d_stores_k(const DevParams& P, int chem) {
+  return !(P.nflow == 4 && ((P.nvars == 11 && (!chem || P.nz == 1)) || P.nvars == 4));
+}
+void launch_stage2d(const DevParams& P, const Stage2D& S, cudaStream_t s);
+// the ghost points of u copied to dst (each of the n states)
+void launch_copy_ghosts(const DevParams& P, const double* u, double* const* dst, int n, cudaStream_t s);
 // the y term of the hyperbolic divergence on a column slab (P: its N0
 // columns, all N1 rows; UT and yi in the transposed layout; dyinv the whole
 // grid's ghosted 1/dy), laid out for the row slabs of n1 rows

@@ -277,15 +277,17 @@ template <typename T> __device__ __forceinline__ T max3v(T a, T b, T c) { return
 //   mode 1: fI = 0.5(fL+fR + alpha(uL-uR))         (LLF, RF mixed)
 //   mode 2: fI = fL ; mode 3: fI = fR               (RF pure upwind)
 // Reference: NavierStokes2DUpwind.c:26-332, Euler1DUpwind.c:27-330.
+// Roe and Rusanov from half the jump ud = (uR - uL) / 2 and the sum sf = fL +
+// fR, with the averages taken between the cell states.
 template <int MODEL, int UPW, typename T>
-__device__ void upwind_flow(const T* uL, const T* uR, const T* fL, const T* fR, const T* uCL,
-                            const T* uCR, T g, int dir, T* fI, T* sp_alpha, int* sp_mode) {
+__device__ __forceinline__ void upwind_cells(const T* ud, const T* sf, const T* uCL, const T* uCR, T g, int dir,
+                                             T* fI, T* sp_alpha, int* sp_mode) {
   typedef Flow<MODEL> F;
   constexpr int NF = F::NF;
   T ua[4], D[4];
+  F::roe_avg(uCL, uCR, g, ua);
   if (UPW == UPW_ROE) {
     T L[4][4], R[4][4];
-    F::roe_avg(uCL, uCR, g, ua);
     T vn = F::eigvals(ua, g, dir, D);
     F::eigvec(ua, g, dir, L, R);
     T Ds[4], dsp;
@@ -300,9 +302,7 @@ __device__ void upwind_flow(const T* uL, const T* uR, const T* fL, const T* fR, 
       for (int a = 0; a < NF; a++) Ds[a] = absv(D[a]);
       dsp = absv(vn);
     }
-    T ud[4], w[4];
-#pragma unroll
-    for (int a = 0; a < NF; a++) ud[a] = T(0.5) * (uR[a] - uL[a]);
+    T w[4];
 #pragma unroll
     for (int a = 0; a < NF; a++) {
       T s = T(0);
@@ -315,11 +315,10 @@ __device__ void upwind_flow(const T* uL, const T* uR, const T* fL, const T* fR, 
       T s = T(0);
 #pragma unroll
       for (int b = 0; b < NF; b++) s += R[a][b] * w[b];
-      fI[a] = T(0.5) * (fL[a] + fR[a]) - s;
+      fI[a] = T(0.5) * sf[a] - s;
     }
-    *sp_alpha = dsp; *sp_mode = 0;
-  } else if (UPW == UPW_RUSANOV) {
-    F::roe_avg(uCL, uCR, g, ua);
+    *sp_alpha = dsp;
+  } else {
     T cL, cR, cA, vL, vR, vA;
     if (MODEL == NS2D) {
       Flow<NS2D>::sound_and_vn(uCL, g, dir, cL, vL);
@@ -335,10 +334,69 @@ __device__ void upwind_flow(const T* uL, const T* uR, const T* fL, const T* fR, 
     }
     T alpha = max3v(cL + absv(vL), cR + absv(vR), cA + absv(vA));
 #pragma unroll
-    for (int a = 0; a < NF; a++) fI[a] = T(0.5) * (fL[a] + fR[a]) - alpha * (T(0.5) * (uR[a] - uL[a]));
-    *sp_alpha = alpha; *sp_mode = 0;
+    for (int a = 0; a < NF; a++) fI[a] = T(0.5) * sf[a] - alpha * ud[a];
+    *sp_alpha = alpha;
+  }
+  *sp_mode = 0;
+}
+
+// Roe, Rusanov or LLF of 2D Navier-Stokes from du = uL - uR and sf = fL + fR
+// (RF needs the separate fluxes).  A, B: the states left and right of the
+// interface the averages and eigenvalues come from -- the cell states (Roe,
+// Rusanov) or the interface states (LLF, in whose deviation form fI = sf / 2
+// + R (|lambda| / 2) L du the mean flux is not projected).
+template <int UPW, typename T>
+__device__ __forceinline__ void ns2d_upwind_packed(const T* A, const T* B, const T* du, const T* sf, T g, int dir,
+                                                   T* fI, T* sp_alpha, int* sp_mode) {
+  constexpr int NF = Flow<NS2D>::NF;
+  if (UPW != UPW_LLF) {
+    T ud[4];
+#pragma unroll
+    for (int a = 0; a < NF; a++) ud[a] = T(-0.5) * du[a];
+    upwind_cells<NS2D, UPW, T>(ud, sf, A, B, g, dir, fI, sp_alpha, sp_mode);
+    return;
+  }
+  T L[4][4], R[4][4], eL[4], eR[4], eC[4], vnL, vnR, vnC;
+  ns2d_char_setup<T>(A, B, g, dir, L, R, eL, eR, eC, vnL, vnR, vnC);
+  T sc[4];
+#pragma unroll
+  for (int a = 0; a < NF; a++) {
+    T d = T(0);
+#pragma unroll
+    for (int b = 0; b < NF; b++) d += L[a][b] * du[b];
+    sc[a] = T(0.5) * max3v(absv(eL[a]), absv(eC[a]), absv(eR[a])) * d;
+  }
+#pragma unroll
+  for (int a = 0; a < NF; a++) {
+    T s = T(0);
+#pragma unroll
+    for (int b = 0; b < NF; b++) s += R[a][b] * sc[b];
+    fI[a] = T(0.5) * sf[a] + s;
+  }
+  *sp_mode = 1;
+  *sp_alpha = max3v(absv(vnL), absv(vnC), absv(vnR));
+}
+
+template <int MODEL, int UPW, typename T>
+__device__ void upwind_flow(const T* uL, const T* uR, const T* fL, const T* fR, const T* uCL,
+                            const T* uCR, T g, int dir, T* fI, T* sp_alpha, int* sp_mode) {
+  typedef Flow<MODEL> F;
+  constexpr int NF = F::NF;
+  T ua[4];
+  if (UPW == UPW_ROE || UPW == UPW_RUSANOV) {
+    T ud[4], sf[4];
+#pragma unroll
+    for (int a = 0; a < NF; a++) { ud[a] = T(0.5) * (uR[a] - uL[a]); sf[a] = fL[a] + fR[a]; }
+    upwind_cells<MODEL, UPW, T>(ud, sf, uCL, uCR, g, dir, fI, sp_alpha, sp_mode);
   } else {
     // characteristic LLF / RF
+    if constexpr (MODEL == NS2D && UPW == UPW_LLF) {
+      T du[4], sf[4];
+#pragma unroll
+      for (int a = 0; a < NF; a++) { du[a] = uL[a] - uR[a]; sf[a] = fL[a] + fR[a]; }
+      ns2d_upwind_packed<UPW, T>(uL, uR, du, sf, g, dir, fI, sp_alpha, sp_mode);
+      return;
+    }
     T L[4][4], R[4][4], eL[4], eR[4], eC[4], vnL, vnR, vnC;
     if (MODEL == NS2D) {
       ns2d_char_setup<T>(uL, uR, g, dir, L, R, eL, eR, eC, vnL, vnR, vnC);

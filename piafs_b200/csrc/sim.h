@@ -25,6 +25,8 @@ struct piafs_gpu_sim {
   cudaStream_t ystream = nullptr;
   cudaEvent_t yfork = nullptr, yjoin = nullptr;
   double* fCy = nullptr;
+  // 2D: the Runge-Kutta combination formed in the kernel that ends a stage
+  bool fuse_rk = false;
   // device state (structure of arrays)
   double* u = nullptr;
   double* U[MAX_STAGES] = {nullptr};       // U[0] aliases u

@@ -131,9 +131,8 @@ int piafs_gpu_slab_create(const char* deck_dir, int precision, int rank, int nra
   C.pis = round32(C.nint[0] > C.nint[1] ? C.nint[0] : C.nint[1]);
   C.jg0 = 0;
   C.N1g = C.N1;
-  // packed passive interface values need every line in one CTA, the column
-  // slab's whole-grid y lines included
-  if (!crweno_line_fits(sl->N1)) s->P.pack_sp = C.pack_sp = 0;
+  // the column slab's whole-grid y lines pack too, or neither slab does
+  if (C.scheme == CRWENO5 && !crweno_packs(sl->N1)) s->P.pack_sp = C.pack_sp = 0;
   sl->PTc = transposed_params(C);
   const size_t planes = (size_t)C.nvars * C.ps, iplanes = (size_t)C.nvars * C.pis;
   const size_t isz = s->P.mixed ? sizeof(float) : sizeof(double);
@@ -252,9 +251,20 @@ int piafs_gpu_slab_stage_end(piafs_gpu_slab* sl, int st) {
   piafs_gpu_sim* s = sl->row;
   const Deck& d = s->deck;
   double* Us = st == 0 ? s->u : s->U[st];
-  const void* xi[4] = {s->iface[0], s->iface[1], s->iface[2], s->iface[3]};
-  launch_upwind_div2d_hy(s->P, Us, xi, s->dxinv, sl->hy_recv, sl->n0, s->Ud[st], 1, s->stream);
-  launch_visc_source(s->P, Us, s->dxinv, s->imap, s->tdev, d.c[st], s->Ud[st], 1, 1, s->stream);
+  Stage2D S{};
+  S.U = Us;
+  for (int k = 0; k < 4; k++) S.xi[k] = s->iface[k];
+  S.hy = sl->hy_recv;
+  S.n0 = sl->n0;
+  S.dxinv = s->dxinv;
+  S.imap = s->imap;
+  S.tdev = s->tdev;
+  S.cstage = d.c[st];
+  S.neg = 1;
+  S.visc = s->P.viscous;
+  S.chem = s->P.chem;
+  S.k = s->Ud[st];
+  launch_stage2d(s->P, S, s->stream);
   SCK(cudaGetLastError());
   return PIAFS_OK;
 }
