@@ -261,8 +261,51 @@ static void enqueue_step(piafs_gpu_sim* s, bool with_norm) {
   launch_advance_time(s->tdev, d.dt, s->stream);
 }
 
+// Steps of a 1D line in launches of many (bounded, so that no launch runs for
+// longer than some milliseconds).
+static int enqueue_run1d(piafs_gpu_sim* s, int nsteps) {
+  for (int k = 0; k < nsteps;) {
+    Run1D R = s->run1d;
+    R.nsteps = std::min(nsteps - k, 1024);
+    CK(launch_run1d(s->P, R, s->run1d_ctas, s->stream));
+    k += R.nsteps;
+  }
+  for (int k = 0; k < nsteps; k++) s->t += s->deck.dt;
+  s->iter += nsteps;
+  return PIAFS_OK;
+}
+
+// the line's arguments for enqueue_run1d, where it is one of those
+static void setup_run1d(piafs_gpu_sim* s) {
+  const DevParams& P = s->P;
+  const Deck& d = s->deck;
+  if (!(P.ndims == 1 && P.model == EULER1D && !P.chem && P.nvars == 3 && P.ghosts == 3 && !P.mixed &&
+        !P.char_interp && s->sponges.empty() && P.N0 >= 16 && d.nstages >= 1))
+    return;
+  Run1D& R = s->run1d;
+  R.u = s->u;
+  R.dxinv = s->dxinv;
+  R.tdev = s->tdev;
+  R.err = s->err;
+  R.nstages = d.nstages;
+  for (int i = 0; i < MAX_STAGES * MAX_STAGES; i++) R.a[i] = d.dt * d.A[i];
+  for (int i = 0; i < MAX_STAGES; i++) R.b[i] = d.dt * d.b[i];
+  for (auto& f : R.face) f = {-1, 0.0, nullptr};
+  for (const Zone& z : d.zones) {
+    if (z.ie[1] <= z.is[1] || z.ie[0] - z.is[0] != P.ghosts) return;   // not a whole face
+    if (!bc_per_variable(z.type) && z.type != BC_SLIPWALL) continue;   // acts in two dimensions only
+    R.face[z.face == 1 ? 0 : 1] = {z.type, z.vel[0], z.val};
+  }
+  s->run1d_ctas = run1d_ctas(P, R);
+}
+
 static int run_steps(piafs_gpu_sim* s, int nsteps, bool norm_last) {
-  for (int k = 0; k < nsteps; k++) {
+  int k0 = 0;
+  if (s->run1d_ctas > 0) {
+    k0 = norm_last ? nsteps - 1 : nsteps;   // a step with the norm: kernel by kernel
+    if (int r = enqueue_run1d(s, k0)) return r;
+  }
+  for (int k = k0; k < nsteps; k++) {
     const bool with_norm = norm_last && (k == nsteps - 1);
     const int gi = with_norm ? 1 : 0;
     if (s->use_graph) {
@@ -430,6 +473,7 @@ int piafs::create_sim(Deck&& deck, int precision, piafs_gpu_sim** out) {
   // one-stage schemes advance u itself, which other tiles still read as the
   // stage's state: their combination stays a kernel of its own
   s->fuse_rk = P.ndims == 2 && !visc4(P) && s->sponges.empty() && d.nstages > 1;
+  setup_run1d(s);
   // initial solution; restart time waqt = restart_iter * dt (TimeInitialize.c:51)
   int rr = piafs_gpu_set_state(s, d.u0.data(), d.restart_iter * d.dt);
   if (rr) { free_sim(s); return rr; }
@@ -475,7 +519,7 @@ int piafs_gpu_get_info(piafs_gpu_sim* s, piafs_gpu_info* info) {
   const int nz = launch_bc(s->P, nullptr, d.zones.data(), (int)d.zones.size(), nullptr);
   const int vs = (((s->P.ndims == 2 && s->P.viscous) || s->P.chem) && (s->P.ndims == 1 || visc4(s->P))) ? 1 : 0;
   const int tr = (s->ut && s->P.model != NS2D) ? 1 : 0;   // NS2D: the transpose also forms the y flux
-  info->launches_per_step = d.nstages * (nz + 2 * s->P.ndims + 1 + tr + vs + (s->fuse_rk ? 0 : 1)) + 1;
+  info->launches_per_step = s->run1d_ctas > 0 ? 1 : d.nstages * (nz + 2 * s->P.ndims + 1 + tr + vs + (s->fuse_rk ? 0 : 1)) + 1;
   return PIAFS_OK;
 }
 
@@ -514,6 +558,11 @@ int piafs_gpu_TimeRK(piafs_gpu_sim* s, int nsteps) {
 
 int piafs_gpu_TimeRK_async(piafs_gpu_sim* s, int nsteps) {
   if (!s || nsteps < 0) return fail(PIAFS_ERR_ARGUMENT, "bad argument");
+  if (s->run1d_ctas > 0) {
+    if (int r = enqueue_run1d(s, nsteps)) return r;
+    CK(cudaGetLastError());
+    return PIAFS_OK;
+  }
   for (int k = 0; k < nsteps; k++) {
     if (s->use_graph) {
       if (!s->graph[0]) {
@@ -774,6 +823,14 @@ static int finish(piafs_gpu_sim* s) {
 
 int piafs_gpu_RHSFunction(piafs_gpu_sim* s, double* rhs, double* u, double t) {
   if (!s || !rhs || !u) return fail(PIAFS_ERR_ARGUMENT, "null argument");
+  if (s->run1d_ctas > 0) {
+    Run1D R = s->run1d;
+    R.u = u;
+    R.rhs = rhs;
+    R.nsteps = 1;
+    CK(launch_run1d(s->P, R, s->run1d_ctas, s->stream));
+    return finish(s);
+  }
   double* U = s->scratch;
   double* R = s->Ud[0];   // its ghost entries are never written: zero
   to_soa(s, u, U);

@@ -258,6 +258,31 @@ void launch_visc_source(const DevParams& P, const double* U, const double* dxinv
                         double* hnu = nullptr);
 void launch_upwind_iface(const DevParams& P, const double* U, const double* uL, const double* uR, const double* fL,
                          const double* fR, double* fI, int dir, cudaStream_t s);
+// Whole time steps of a 1D Euler line in one launch (run1d.cu): components,
+// FP64, three variables, at least 16 points.  face[k]: what
+// sets the ghosts of the left (0) and right (1) end -- the last zone of that
+// face that acts in one dimension (type -1: none, the ghosts keep their
+// values); the other fields as in Zone.  With rhs: one evaluation of the
+// right-hand side instead, u and rhs point-major with ghosts.
+struct Run1D {
+  double* u;
+  double* rhs;
+  const double* dxinv;
+  double* tdev;
+  int* err;                            // set on a zero pivot (CRWENO5)
+  int nstages, nsteps;
+  double a[MAX_STAGES * MAX_STAGES];   // dt * A
+  double b[MAX_STAGES];                // dt * b
+  struct Face { int type; double vel; const double* val; } face[2];
+};
+constexpr int kRun1DSmem = 200 * 1024;
+constexpr int kRun1DCrwSmem = 222 * 1024;
+// the CTAs (one cluster) that run a line, 0 if it does not fit; CRWENO5 lines
+// of up to 8193 points in run1d_crw.cu
+int run1d_crw_ctas(const DevParams& P, const Run1D& R);
+cudaError_t launch_run1d_crw(const DevParams& P, const Run1D& R, int ctas, cudaStream_t s);
+int run1d_ctas(const DevParams& P, const Run1D& R);
+cudaError_t launch_run1d(const DevParams& P, const Run1D& R, int ctas, cudaStream_t s);
 void launch_first_deriv(const DevParams& P, double* Df, const double* f, int dir, int bias, int nv, cudaStream_t s);
 void launch_advance_time(double* tdev, double dt, cudaStream_t s);
 void launch_reciprocal(const double* x, double* y, long long n, cudaStream_t s);

@@ -27,6 +27,10 @@ struct piafs_gpu_sim {
   double* fCy = nullptr;
   // 2D: the Runge-Kutta combination formed in the kernel that ends a stage
   bool fuse_rk = false;
+  // 1D Euler lines whose steps run in one launch: its arguments and CTAs (0:
+  // the kernels one by one)
+  Run1D run1d{};
+  int run1d_ctas = 0;
   // device state (structure of arrays)
   double* u = nullptr;
   double* U[MAX_STAGES] = {nullptr};       // U[0] aliases u
