@@ -154,6 +154,75 @@ __global__ void __launch_bounds__(256) k_transpose_flux_y(DevParams P, const dou
   }
 }
 
+// The same for grids of few tiles: a block per tile and part, part 0 the flow
+// variables and their flux, every other part one passive variable and its flux
+// vn U_m, for which it reads the density and momentum again.  On the nine tiles
+// of a 64^2 grid k_transpose_flux_y, whose blocks run a tile's variables one
+// after another with two barriers each, took 18 us of latency, and a step 95
+// us where it takes 83 with the variables in blocks of their own; where the
+// tiles fill the GPU the second reading costs more than the barriers (512^2: 33
+// against 29 us, 2048^2: 353 against 279).
+__global__ void __launch_bounds__(256) k_transpose_flux_y_parts(DevParams P, const double* __restrict__ U,
+                                                          double* __restrict__ UT, double* __restrict__ FT) {
+  __shared__ double tile[4][32][33];
+  const int W0 = P.W0, W1 = P.W1, parts = P.nvars - 3, part = blockIdx.x % parts;
+  const long long ps = P.ps;
+  const int i0 = blockIdx.x / parts * 32, j0 = blockIdx.y * 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  if (part > 0) {
+    const int m = 3 + part;
+    double x[4], r[4], v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int i = i0 + tx, j = j0 + ty + 8 * k;
+      const bool in = i < W0 && j < W1;
+      const long long p = (long long)j * W0 + i;
+      x[k] = in ? U[m * ps + p] : 0.0;
+      r[k] = in ? U[p] : 0.0;
+      v[k] = in ? U[2 * ps + p] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      tile[0][ty + 8 * k][tx] = x[k];
+      tile[1][ty + 8 * k][tx] = __dmul_rn(r[k] == 0.0 ? 0.0 : v[k] / r[k], x[k]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int i = i0 + ty + 8 * k, j = j0 + tx;
+      if (i < W0 && j < W1) {
+        const long long q = (long long)i * W1 + j;
+        UT[m * ps + q] = tile[0][tx][ty + 8 * k];
+        FT[m * ps + q] = tile[1][tx][ty + 8 * k];
+      }
+    }
+    return;
+  }
+#pragma unroll
+  for (int m = 0; m < 4; m++)
+    for (int r = ty; r < 32; r += 8) {
+      const int i = i0 + tx, j = j0 + r;
+      if (i < W0 && j < W1) tile[m][r][tx] = U[m * ps + (long long)j * W0 + i];
+    }
+  __syncthreads();
+  // point (i = i0 + r, j = j0 + tx): writes along j are coalesced
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int r = ty + 8 * k;
+    const int j = j0 + tx, i = i0 + r;
+    if (i < W0 && j < W1) {
+      double f[4], vn;
+      ns2d_flux(tile[0][tx][r], tile[1][tx][r], tile[2][tx][r], tile[3][tx][r], P.gamma, 1, f, vn);
+      const long long q = (long long)i * W1 + j;
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        UT[m * ps + q] = tile[m][tx][r];
+        FT[m * ps + q] = f[m];
+      }
+    }
+  }
+}
+
 // The ghost points of a state copied to others: entry v of a ghost that no
 // boundary zone writes (corners; the passive variables at walls) keeps its
 // value through a step, in the stage states too.
@@ -935,8 +1004,11 @@ void launch_iface_soa_to_aos(const double* soa, double* aos, long long ni, int n
   point_major<false, false>(DevParams{}, aos, const_cast<double*>(soa), ni, nv, pis, s);
 }
 void launch_transpose_flux_y(const DevParams& P, const double* U, double* UT, double* FT, cudaStream_t s) {
-  dim3 grid(nblk(P.W0, 32), nblk(P.W1, 32)), blk(32, 8);
-  k_transpose_flux_y<<<grid, blk, 0, s>>>(P, U, UT, FT);
+  const unsigned tx = nblk(P.W0, 32), ty = nblk(P.W1, 32);
+  const dim3 blk(32, 8);
+  // up to one tile an SM the tiles' variables in blocks of their own
+  if (tx * ty <= 148 && P.nvars > 4) k_transpose_flux_y_parts<<<dim3(tx * (P.nvars - 3), ty), blk, 0, s>>>(P, U, UT, FT);
+  else k_transpose_flux_y<<<dim3(tx, ty), blk, 0, s>>>(P, U, UT, FT);
 }
 void launch_transpose(const DevParams& P, const double* in, double* out, cudaStream_t s) {
   dim3 grid(nblk(P.W0, 32), nblk(P.W1, 32), P.nvars), blk(32, 8);
