@@ -71,55 +71,55 @@ static void free_sim(piafs_gpu_sim* s) {
 }
 
 // -------------------------------------------------------------- the RHS
-// Cell-centred flux and interface values (uL, uR, fL, fR into I) of
-// direction d.  The y pass of a 2D CRWENO5 run works on a transposed copy of
-// U so that its lines, the tridiagonal systems, are contiguous in memory; its
-// interface arrays are then in the transposed layout.  If `ev` is given, an
-// event is recorded after the flux and after the reconstruction.
-void piafs::enqueue_recon(piafs_gpu_sim* s, const double* U, int d, double* const* I, cudaEvent_t* ev, int* k) {
+// Cell-centred flux (into F) and interface values (uL, uR, fL, fR into I) of
+// direction d, on the given stream.  The y pass of a 2D CRWENO5 run works on a
+// transposed copy of U so that its lines, the tridiagonal systems, are
+// contiguous in memory; its interface arrays are then in the transposed layout.
+// If `ev` is given, an event is recorded after the flux and after the
+// reconstruction.
+static void enqueue_recon_on(piafs_gpu_sim* s, const double* U, int d, double* F, double* const* I, cudaStream_t st,
+                             cudaEvent_t* ev, int* k) {
   const DevParams& P = s->P;
-  auto mark = [&]() { if (ev) cudaEventRecord(ev[++*k], s->stream); };
-  if (P.scheme == CRWENO5 && P.char_interp) {
-    launch_flux(P, U, s->fC, d, s->stream);
-    mark();
-    launch_crweno_char(P, U, s->fC, I[0], I[1], I[2], I[3], d, s->crwchar, s->err, s->stream);
-    mark();
-    return;
-  }
+  auto mark = [&]() { if (ev) cudaEventRecord(ev[++*k], st); };
   if (d == 1 && s->ut) {
     if (P.model == NS2D) {
-      launch_transpose_flux_y(P, U, s->ut, s->fC, s->stream);
+      launch_transpose_flux_y(P, U, s->ut, F, st);
     } else {
-      launch_transpose(P, U, s->ut, s->stream);
-      launch_flux(P, s->ut, s->fC, 1, s->stream);
+      launch_transpose(P, U, s->ut, st);
+      launch_flux(P, s->ut, F, 1, st);
     }
     mark();
-    launch_crweno(s->PT, s->ut, s->fC, I[0], I[1], I[2], I[3], 0, s->err, s->stream);
+    launch_crweno(s->PT, s->ut, F, I[0], I[1], I[2], I[3], 0, s->err, st);
     mark();
     return;
   }
-  launch_flux(P, U, s->fC, d, s->stream);
+  launch_flux(P, U, F, d, st);
   mark();
-  if (P.scheme != CRWENO5 && P.char_interp) launch_weno5_char(P, U, s->fC, I[0], I[1], I[2], I[3], d, s->stream);
-  else if (P.scheme != CRWENO5) launch_weno5(P, U, s->fC, I[0], I[1], I[2], I[3], d, s->stream);
-  else launch_crweno(P, U, s->fC, I[0], I[1], I[2], I[3], d, s->err, s->stream);
+  if (P.scheme == CRWENO5 && P.char_interp)
+    launch_crweno_char(P, U, F, I[0], I[1], I[2], I[3], d, s->crwchar, s->err, st);
+  else if (P.scheme != CRWENO5 && P.char_interp) launch_weno5_char(P, U, F, I[0], I[1], I[2], I[3], d, st);
+  else if (P.scheme != CRWENO5) launch_weno5(P, U, F, I[0], I[1], I[2], I[3], d, st);
+  else launch_crweno(P, U, F, I[0], I[1], I[2], I[3], d, s->err, st);
   mark();
 }
 
+void piafs::enqueue_recon(piafs_gpu_sim* s, const double* U, int d, double* const* I, cudaEvent_t* ev, int* k) {
+  enqueue_recon_on(s, U, d, s->fC, I, s->stream, ev, k);
+}
+
 // The reconstruction of both directions of a 2D grid: the y pass on its own
-// stream, concurrent with the x pass, where the simulation has one (and no
-// phase events are asked for); joined when this returns.
+// stream and flux array, concurrent with the x pass, where the simulation has
+// one (and no phase events are asked for); joined when this returns.  On small
+// and middling grids neither pass fills the GPU: the 300 x 217 WENO5 step took
+// 148 us with the passes in turn, 141 with both at once.
 static void enqueue_recon2d(piafs_gpu_sim* s, const double* U, cudaEvent_t* ev = nullptr, int* k = nullptr) {
-  const DevParams& P = s->P;
   const bool concurrent = s->concurrent_y && !ev;
   if (concurrent) cudaEventRecord(s->yfork, s->stream);
   enqueue_recon(s, U, 0, s->iface, ev, k);
   if (concurrent) {
     // the y pass joins the x pass's stream before the kernel that ends the stage
     cudaStreamWaitEvent(s->ystream, s->yfork, 0);
-    double* const* Iy = s->iface_y;
-    launch_transpose_flux_y(P, U, s->ut, s->fCy, s->ystream);
-    launch_crweno(s->PT, s->ut, s->fCy, Iy[0], Iy[1], Iy[2], Iy[3], 0, s->err, s->ystream);
+    enqueue_recon_on(s, U, 1, s->fCy, s->iface_y, s->ystream, nullptr, nullptr);
     cudaEventRecord(s->yjoin, s->ystream);
     cudaStreamWaitEvent(s->stream, s->yjoin, 0);
   } else {
@@ -412,16 +412,18 @@ int piafs::create_sim(Deck&& deck, int precision, piafs_gpu_sim** out) {
       (P.mixed || !(noyt && noyt[0] == '1'))) {
     e = alloc(&s->ut, planes);
     s->PT = transposed_params(P);
-    // PIAFS_GPU_NO_CONCURRENT_Y=1 runs the y pass after the x pass on one
-    // stream (the same values)
-    const char* ncy = std::getenv("PIAFS_GPU_NO_CONCURRENT_Y");
-    if (e == cudaSuccess && P.model == NS2D && !(ncy && ncy[0] == '1')) {
-      e = alloc(&s->fCy, planes);
-      if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->ystream, cudaStreamNonBlocking);
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->yfork, cudaEventDisableTiming);
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->yjoin, cudaEventDisableTiming);
-      s->concurrent_y = e == cudaSuccess;
-    }
+  }
+  // The y pass on a stream of its own (2D Navier-Stokes; the characteristic
+  // CRWENO5 solves share one scratch).  PIAFS_GPU_NO_CONCURRENT_Y=1 runs it
+  // after the x pass on one stream (the same values).
+  const char* ncy = std::getenv("PIAFS_GPU_NO_CONCURRENT_Y");
+  if (e == cudaSuccess && P.ndims == 2 && P.model == NS2D && !s->crwchar &&
+      (P.scheme != CRWENO5 || s->ut) && !(ncy && ncy[0] == '1')) {
+    e = alloc(&s->fCy, planes);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->ystream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->yfork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->yjoin, cudaEventDisableTiming);
+    s->concurrent_y = e == cudaSuccess;
   }
   if (e == cudaSuccess) e = alloc(&s->dxinv, d.dxinv.size());
   if (e == cudaSuccess) e = alloc(&s->imap, d.imap.size());
@@ -837,7 +839,7 @@ int piafs_gpu_RHSFunction(piafs_gpu_sim* s, double* rhs, double* u, double t) {
   enqueue_bc(s, U);
   if (int r = set_top_t(s, t)) return r;
   enqueue_rhs(s, R, U, s->top_t, 0.0);
-  launch_soa_to_aos(U, u, s->P.npg, s->P.nvars, s->P.ps, s->stream);
+  launch_ghosts_to_aos(s->P, U, u, s->stream);   // all that changed in u
   launch_soa_to_aos(R, rhs, s->P.npg, s->P.nvars, s->P.ps, s->stream);
   return finish(s);
 }
@@ -877,7 +879,7 @@ int piafs_gpu_ApplyBoundaryConditions(piafs_gpu_sim* s, double* u, double) {
   if (!s || !u) return fail(PIAFS_ERR_ARGUMENT, "null argument");
   to_soa(s, u, s->scratch);
   enqueue_bc(s, s->scratch);
-  launch_soa_to_aos(s->scratch, u, s->P.npg, s->P.nvars, s->P.ps, s->stream);
+  launch_ghosts_to_aos(s->P, s->scratch, u, s->stream);
   return finish(s);
 }
 

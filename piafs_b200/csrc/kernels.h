@@ -240,6 +240,8 @@ inline bool stage2d_stores_k(const DevParams& P, int chem) {
   return !(P.nflow == 4 && ((P.nvars == 11 && (!chem || P.nz == 1)) || P.nvars == 4));
 }
 void launch_stage2d(const DevParams& P, const Stage2D& S, cudaStream_t s);
+// the ghost points of a state copied to their places of a point-major array
+void launch_ghosts_to_aos(const DevParams& P, const double* soa, double* aos, cudaStream_t s);
 // the ghost points of u copied to dst (each of the n states)
 void launch_copy_ghosts(const DevParams& P, const double* u, double* const* dst, int n, cudaStream_t s);
 // the y term of the hyperbolic divergence on a column slab (P: its N0
