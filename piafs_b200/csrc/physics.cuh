@@ -180,7 +180,10 @@ __device__ __forceinline__ void euler1d_flux(double u0, double u1, double u2, do
 // Reciprocal in the working precision: rcp_nr (common.cuh) for both types.
 template <typename T> __device__ __forceinline__ T rcpw(T x) { return rcp_nr(x); }
 
-// The characteristic-upwinding set-up of 2D Navier-Stokes at one interface
+// The characteristic-upwinding set-up of 2D Navier-Stokes at one interface in
+// matrix form, for RF: its pure-upwind branch R (L f) carries the rounding of
+// the products, which solutions of the compact scheme amplify (1e-14 to 1e-12
+// in sixty steps), so it is formed as the reference forms it
 // (NavierStokes2DUpwind.c:190-260 / 271-332): the Roe average of the two
 // interface states (_NavierStokes2DRoeAverage_, navierstokes2d.h:115-159),
 // its left / right eigenvectors (_NavierStokes2DLeftEigenvectors_ /
@@ -265,6 +268,81 @@ __device__ __forceinline__ void ns2d_char_setup(const T* uL, const T* uR, T g, i
   }
 }
 
+// The characteristic fields of 2D Navier-Stokes at one interface
+// (NavierStokes2DUpwind.c:190-260 / 271-332) in closed form: the averaged
+// state's normal and tangential velocity, sound speed, kinetic energy and
+// enthalpy, from which left() projects a vector on the left eigenvectors
+// (_NavierStokes2DLeftEigenvectors_, navierstokes2d.h:194-252) and right()
+// maps characteristic amplitudes back (_RightEigenvectors_, :254-313).  The
+// fields are ordered un - a, un, un + a, and the shear wave (speed un; its
+// eigenvectors with the opposite sign in x, which cancels).  The products of
+// the 4 x 4 matrices reduce to a pressure and a velocity jump: 12 operations a
+// vector where a matrix takes 16, and seven values kept where two matrices are
+// 32, which decides how many threads an SM holds.
+template <typename T>
+struct NsFields {
+  T un, ut, a, ek, h0, gm1, ia2;
+  __device__ __forceinline__ void set(T un_, T ut_, T a_, T H, T ek_, T gm1_) {
+    un = un_; ut = ut_; a = a_; ek = ek_; h0 = H; gm1 = gm1_;
+    ia2 = rcpw(a_ * a_);
+  }
+  __device__ __forceinline__ void left(const T* X, int dir, T* w) const {
+    const T n = dir == 0 ? X[1] : X[2], t = dir == 0 ? X[2] : X[1];
+    const T dp = gm1 * (ek * X[0] - un * n - ut * t + X[3]), adu = a * (n - un * X[0]), i2a2 = T(0.5) * ia2;
+    w[0] = (dp - adu) * i2a2;
+    w[1] = X[0] - dp * ia2;
+    w[2] = (dp + adu) * i2a2;
+    w[3] = t - ut * X[0];
+  }
+  // f + the vector of the amplitudes w
+  __device__ __forceinline__ void right(const T* w, int dir, T* f) const {
+    const T s = w[0] + w[2], d = a * (w[2] - w[0]), all = s + w[1];
+    f[0] += all;
+    f[dir == 0 ? 1 : 2] += un * all + d;
+    f[dir == 0 ? 2 : 1] += ut * all + w[3];
+    f[3] += h0 * s + un * d + ek * w[1] + ut * w[3];
+  }
+};
+
+// The fields of the Roe average of the two interface states
+// (_NavierStokes2DRoeAverage_, navierstokes2d.h:115-159) and the normal
+// velocities and sound speeds of both states (_NavierStokes2DEigenvalues_,
+// :161-190): each state's velocity, pressure and sound speed formed once and
+// shared, quotients as products with one reciprocal (rcp_nr) -- 4 reciprocals
+// and 5 square roots per interface where the per-macro form takes 25
+// divisions and 7 roots.  The results agree with the macro form to rounding.
+template <typename T>
+__device__ __forceinline__ void ns2d_fields(const T* uL, const T* uR, T g, int dir, NsFields<T>& F, T& vnL, T& cL,
+                                            T& vnR, T& cR) {
+  const T gm1 = g - T(1), igm1 = rcpw(gm1);
+  // one side: velocity, pressure (_NavierStokes2DGetFlowVar_,
+  // navierstokes2d.h:70-80), c^2 = gamma P / rho, enthalpy
+  auto side = [&](const T* u, T& vx, T& vy, T& csq, T& H) {
+    const T rho = u[0];
+    const T ir = rho == T(0) ? T(0) : rcpw(rho);
+    vx = u[1] * ir;
+    vy = u[2] * ir;
+    const T vsq = vx * vx + vy * vy;
+    const T P = (u[3] - T(0.5) * rho * vsq) * gm1;
+    csq = g * P * ir;
+    H = T(0.5) * vsq + csq * igm1;
+  };
+  T vxL, vyL, cLsq, HL, vxR, vyR, cRsq, HR;
+  side(uL, vxL, vyL, cLsq, HL);
+  side(uR, vxR, vyR, cRsq, HR);
+  cL = sqrt(cLsq);
+  cR = sqrt(cRsq);
+  vnL = dir == 0 ? vxL : vyL;
+  vnR = dir == 0 ? vxR : vyR;
+  const T tL = sqrt(uL[0]), tR = sqrt(uR[0]);
+  const T inv = rcpw(tL + tR);
+  const T vx = (tL * vxL + tR * vxR) * inv, vy = (tL * vyL + tR * vyR) * inv;
+  const T H = (tL * HL + tR * HR) * inv;
+  const T ek = T(0.5) * (vx * vx + vy * vy);
+  const T a = sqrt(gm1 * (H - ek));
+  F.set(dir == 0 ? vx : vy, dir == 0 ? vy : vx, a, a * a * igm1 + ek, ek, gm1);
+}
+
 template <typename T> __device__ __forceinline__ T absv(T a) { return a < T(0) ? -a : a; }
 template <typename T> __device__ __forceinline__ T maxv(T a, T b) { return a > b ? a : b; }
 template <typename T> __device__ __forceinline__ T max3v(T a, T b, T c) { return maxv(maxv(a, b), maxv(b, c)); }
@@ -285,23 +363,32 @@ __device__ __forceinline__ void upwind_cells(const T* ud, const T* sf, const T* 
   typedef Flow<MODEL> F;
   constexpr int NF = F::NF;
   T ua[4], D[4];
+  if constexpr (MODEL == NS2D && UPW == UPW_ROE) {
+    // the cells' average; entropy fix, delta = 1e-6 (NavierStokes2DUpwind.c:75-78)
+    NsFields<T> C;
+    T vnL, cL, vnR, cR, w[4];
+    ns2d_fields<T>(uCL, uCR, g, dir, C, vnL, cL, vnR, cR);
+    const T delta = T(0.000001), delta2 = delta * delta, i2d = T(1) / (T(2) * delta);
+    auto fix = [&](T x) { return absv(x) < delta ? (x * x + delta2) * i2d : absv(x); };
+    C.left(ud, dir, w);
+    const T d0 = fix(C.un);
+    w[0] *= -fix(C.un - C.a); w[1] *= -d0; w[2] *= -fix(C.un + C.a); w[3] *= -d0;
+#pragma unroll
+    for (int k = 0; k < NF; k++) fI[k] = T(0.5) * sf[k];
+    C.right(w, dir, fI);
+    *sp_alpha = d0;
+    *sp_mode = 0;
+    return;
+  }
   F::roe_avg(uCL, uCR, g, ua);
   if (UPW == UPW_ROE) {
     T L[4][4], R[4][4];
     T vn = F::eigvals(ua, g, dir, D);
     F::eigvec(ua, g, dir, L, R);
-    T Ds[4], dsp;
-    if (MODEL == NS2D) {
-      // entropy fix, delta = 1e-6 (NavierStokes2DUpwind.c:75-78)
-      const T delta = T(0.000001), delta2 = delta * delta, i2d = T(1) / (T(2) * delta);
+    T Ds[4];
+    const T dsp = absv(vn);
 #pragma unroll
-      for (int a = 0; a < NF; a++) Ds[a] = absv(D[a]) < delta ? (D[a] * D[a] + delta2) * i2d : absv(D[a]);
-      dsp = absv(vn) < delta ? (vn * vn + delta2) * i2d : absv(vn);
-    } else {
-#pragma unroll
-      for (int a = 0; a < NF; a++) Ds[a] = absv(D[a]);
-      dsp = absv(vn);
-    }
+    for (int a = 0; a < NF; a++) Ds[a] = absv(D[a]);
     T w[4];
 #pragma unroll
     for (int a = 0; a < NF; a++) {
@@ -356,25 +443,19 @@ __device__ __forceinline__ void ns2d_upwind_packed(const T* A, const T* B, const
     upwind_cells<NS2D, UPW, T>(ud, sf, A, B, g, dir, fI, sp_alpha, sp_mode);
     return;
   }
-  T L[4][4], R[4][4], eL[4], eR[4], eC[4], vnL, vnR, vnC;
-  ns2d_char_setup<T>(A, B, g, dir, L, R, eL, eR, eC, vnL, vnR, vnC);
-  T sc[4];
+  NsFields<T> F;
+  T vnL, cL, vnR, cR, w[4];
+  ns2d_fields<T>(A, B, g, dir, F, vnL, cL, vnR, cR);
+  F.left(du, dir, w);
+  const T am = T(0.5) * max3v(absv(vnL - cL), absv(F.un - F.a), absv(vnR - cR));
+  const T ap = T(0.5) * max3v(absv(vnL + cL), absv(F.un + F.a), absv(vnR + cR));
+  const T a0 = max3v(absv(vnL), absv(F.un), absv(vnR));
+  w[0] *= am; w[1] *= T(0.5) * a0; w[2] *= ap; w[3] *= T(0.5) * a0;
 #pragma unroll
-  for (int a = 0; a < NF; a++) {
-    T d = T(0);
-#pragma unroll
-    for (int b = 0; b < NF; b++) d += L[a][b] * du[b];
-    sc[a] = T(0.5) * max3v(absv(eL[a]), absv(eC[a]), absv(eR[a])) * d;
-  }
-#pragma unroll
-  for (int a = 0; a < NF; a++) {
-    T s = T(0);
-#pragma unroll
-    for (int b = 0; b < NF; b++) s += R[a][b] * sc[b];
-    fI[a] = T(0.5) * sf[a] + s;
-  }
+  for (int k = 0; k < NF; k++) fI[k] = T(0.5) * sf[k];
+  F.right(w, dir, fI);
   *sp_mode = 1;
-  *sp_alpha = max3v(absv(vnL), absv(vnC), absv(vnR));
+  *sp_alpha = a0;
 }
 
 template <int MODEL, int UPW, typename T>
@@ -458,16 +539,39 @@ __device__ void upwind_flow_dev(const T* uL, const T* uR, const T* fL, const T* 
     upwind_flow<MODEL, UPW, T>(uL, uR, fL, fR, uCL, uCR, g, dir, fI, sp_alpha, sp_mode);
     return;
   }
-  T ua[4], L[4][4], R[4][4], eL[4], eR[4], eC[4], vnL, vnR, vnC;
-  if (MODEL == NS2D) {
-    ns2d_char_setup<T>(uAL, uAR, g, dir, L, R, eL, eR, eC, vnL, vnR, vnC);
-  } else {
-    F::roe_avg(uCL, uCR, g, ua);
-    F::eigvec(ua, g, dir, L, R);
-    vnL = F::eigvals(uCL, g, dir, eL);
-    vnR = F::eigvals(uCR, g, dir, eR);
-    vnC = F::eigvals(ua, g, dir, eC);
+  if constexpr (MODEL == NS2D) {
+    NsFields<T> C;
+    T vnL, cL, vnR, cR, wu[4], wf[4], du[4], df[4];
+    ns2d_fields<T>(uAL, uAR, g, dir, C, vnL, cL, vnR, cR);
+#pragma unroll
+    for (int k = 0; k < NF; k++) {
+      du[k] = uL[k] - uR[k];
+      df[k] = fL[k] - fR[k];
+      fI[k] = T(0.5) * (fL[k] + fR[k]);
+    }
+    C.left(du, dir, wu);
+    C.left(df, dir, wf);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const T o = k == 0 ? T(-1) : k == 2 ? T(1) : T(0);   // the field's speed is vn + o c
+      const T l = vnL + o * cL, m = C.un + o * C.a, r = vnR + o * cR;
+      if (UPW == UPW_RF && l > T(0) && m > T(0) && r > T(0)) wu[k] = T(0.5) * wf[k];
+      else if (UPW == UPW_RF && l < T(0) && m < T(0) && r < T(0)) wu[k] = T(-0.5) * wf[k];
+      else wu[k] *= T(0.5) * max3v(absv(l), absv(m), absv(r));
+    }
+    C.right(wu, dir, fI);
+    if (UPW == UPW_RF && vnL > T(0) && C.un > T(0) && vnR > T(0)) *sp_mode = 2;
+    else if (UPW == UPW_RF && vnL < T(0) && C.un < T(0) && vnR < T(0)) *sp_mode = 3;
+    else *sp_mode = 1;
+    *sp_alpha = max3v(absv(vnL), absv(C.un), absv(vnR));
+    return;
   }
+  T ua[4], L[4][4], R[4][4], eL[4], eR[4], eC[4], vnL, vnR, vnC;
+  F::roe_avg(uCL, uCR, g, ua);
+  F::eigvec(ua, g, dir, L, R);
+  vnL = F::eigvals(uCL, g, dir, eL);
+  vnR = F::eigvals(uCR, g, dir, eR);
+  vnC = F::eigvals(ua, g, dir, eC);
   T sc[4];
 #pragma unroll
   for (int a = 0; a < NF; a++) {

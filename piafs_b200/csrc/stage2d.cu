@@ -38,10 +38,18 @@ constexpr int QX = TI + 2, QY = TJ + 2, FX = TI + 1, FY = TJ + 1;
 // interfaces but the y term itself (a grid decomposed along y)
 enum YMode { Y_STD = 0, Y_TRANSPOSED = 1, Y_GIVEN = 2 };
 
+// CTAs an SM: registers for two 128, three 80, four 64.  Mixed precision four
+// (701 x 500: 54.9 us, 62.8 with three); FP64 three (64 registers spill: LLF at
+// 2048 x 2048 takes 940 us with four, 703 with three; Roe at 300 x 217 22.1 and
+// 18.4); RF's matrices in FP64 two (1201 x 777: 131.1 us, 133.3 with three).
+constexpr int stage2d_ctas(int upw, bool mx) { return mx ? 4 : upw == UPW_RF ? 2 : 3; }
+
 template <typename T>
 constexpr size_t stage2d_smem(int nv, bool given, bool visc) {
-  return ((size_t)nv * (NX + (given ? 0 : NY)) + (visc ? 2 * QX * QY + 3 * TJ * FX + 3 * FY * TI : 0)) * sizeof(T) +
-         (visc ? QX * QY * sizeof(double) : 0);
+  // interface fluxes, after velocities and temperature in the same place; the
+  // viscous fluxes
+  const size_t hyp = (size_t)nv * (NX + (given ? 0 : NY)) * sizeof(T), q = QX * QY * (2 * sizeof(T) + sizeof(double));
+  return visc ? (3 * TJ * FX + 3 * FY * TI) * sizeof(T) + (hyp > q ? hyp : q) : hyp;
 }
 
 // Upwind flux of all components at interface q into so[m * stride]; cells pL
@@ -138,7 +146,7 @@ __device__ __forceinline__ void iface_upwind(const DevParams& P, const void* __r
 // NV: the number of variables when it is 11 (one chemistry layer) or 4 (none),
 // 0 for any other: the registers hold the point's variables group by group.
 template <int UPW, int YM, bool MX, int NV>
-__global__ void __launch_bounds__(256, UPW == UPW_RF && !MX ? 2 : 3) k_stage2d(DevParams P, Stage2D S) {
+__global__ void __launch_bounds__(256, stage2d_ctas(UPW, MX)) k_stage2d(DevParams P, Stage2D S) {
   typedef typename std::conditional<MX, float, double>::type T;
   extern __shared__ double sfd[];
   constexpr bool GIVEN = YM == Y_GIVEN;
@@ -149,14 +157,15 @@ __global__ void __launch_bounds__(256, UPW == UPW_RF && !MX ? 2 : 3) k_stage2d(D
   const int i0 = blockIdx.x * TI, j0 = blockIdx.y * TJ;
   const int tid = threadIdx.x;
   const bool visc = S.visc != 0;
-  // the temperature on the tile and one cell around it [QY][QX], FP64 also in
-  // mixed precision: its differences are taken before they are rounded
-  double* sT_ = sfd;
-  T* sQ = (T*)(sfd + (visc ? QX * QY : 0));   // u, v there [2][QY][QX]
-  T* sVx = sQ + (visc ? 2 * QX * QY : 0);     // viscous x fluxes [3][TJ][FX]
+  T* sVx = (T*)sfd;                           // viscous x fluxes [3][TJ][FX]
   T* sVy = sVx + (visc ? 3 * TJ * FX : 0);    // viscous y fluxes [3][FY][TI]
   T* sx = sVy + (visc ? 3 * FY * TI : 0);     // x-interface fluxes [m][row jj][ii = 0..TI]
   T* sy = sx + nv * NX;                       // y-interface fluxes [m][column ii][jj = 0..TJ]
+  // before the interface fluxes, in their place: the temperature on the tile
+  // and one cell around it [QY][QX], FP64 also in mixed precision (its
+  // differences are taken before they are rounded), and u, v [2][QY][QX]
+  double* sT_ = (double*)sx;
+  T* sQ = (T*)(sT_ + QX * QY);
   if (visc) {
     for (int e = tid; e < QX * QY; e += 256) {
       const int a = e % QX, b = e / QX;
@@ -170,46 +179,7 @@ __global__ void __launch_bounds__(256, UPW == UPW_RF && !MX ? 2 : 3) k_stage2d(D
       }
       sQ[e] = (T)uu; sQ[QX * QY + e] = (T)vv; sT_[e] = TT;
     }
-  }
-  double uref[4];
-  if (tid < NX) {                // (TI + 1) x TJ x interfaces
-    const int ii = tid % LX, jj = tid / LX;
-    const int i = i0 + ii, j = j0 + jj;
-    if (i <= N0 && j < N1) {
-      const long long pR = pidx(P, i, j);
-      if (MX && (UPW == UPW_LLF || UPW == UPW_RF)) {
-        const long long p0 = pidx(P, 0, j);
-#pragma unroll
-        for (int m = 0; m < 4; m++) uref[m] = U[m * ps + p0];
-      }
-      iface_upwind<UPW, 0, MX>(P, S.xi[0], S.xi[1], S.xi[2], S.xi[3], i + (long long)(N0 + 1) * j, U, pR - 1, pR,
-                               uref, sx + jj * LX + ii, NX);
-    }
-  }
-  if (!GIVEN && tid < NY) {      // TI x (TJ + 1) y interfaces
-    int ii, jj;
-    if (YM == Y_TRANSPOSED) { jj = tid % LY; ii = tid / LY; }
-    else { ii = tid % TI; jj = tid / TI; }
-    const int i = i0 + ii, j = j0 + jj;
-    if (j <= N1 && i < N0) {
-      if (MX && (UPW == UPW_LLF || UPW == UPW_RF)) {
-        const long long p0 = pidx(P, i, 0);
-#pragma unroll
-        for (int m = 0; m < 4; m++) uref[m] = U[m * ps + p0];
-      }
-      if (YM == Y_TRANSPOSED) {
-        const long long pR = (long long)(j + g) + (long long)P.W1 * (i + g);
-        iface_upwind<UPW, 1, MX>(P, S.yi[0], S.yi[1], S.yi[2], S.yi[3], j + (long long)(N1 + 1) * i, S.UT, pR - 1,
-                                 pR, uref, sy + ii * LY + jj, NY);
-      } else {
-        const long long pR = pidx(P, i, j);
-        iface_upwind<UPW, 1, MX>(P, S.yi[0], S.yi[1], S.yi[2], S.yi[3], i + (long long)N0 * j, U, pR - P.W0, pR,
-                                 uref, sy + ii * LY + jj, NY);
-      }
-    }
-  }
-  __syncthreads();
-  if (visc) {
+    __syncthreads();
     const T two_third = T(2.0 / 3.0), inv_Re = (T)(1.0 / P.Re), inv_Pr = (T)(1.0 / P.Pr);
     const T igm1 = (T)(1.0 / (P.gamma - 1.0));
     // viscous fluxes on [i0-1, i0+TI) x [j0-1, j0+TJ) (corner cell unused)
@@ -253,6 +223,44 @@ __global__ void __launch_bounds__(256, UPW == UPW_RF && !MX ? 2 : 3) k_stage2d(D
     }
     __syncthreads();
   }
+  double uref[4];
+  if (tid < NX) {                // (TI + 1) x TJ x interfaces
+    const int ii = tid % LX, jj = tid / LX;
+    const int i = i0 + ii, j = j0 + jj;
+    if (i <= N0 && j < N1) {
+      const long long pR = pidx(P, i, j);
+      if (MX && (UPW == UPW_LLF || UPW == UPW_RF)) {
+        const long long p0 = pidx(P, 0, j);
+#pragma unroll
+        for (int m = 0; m < 4; m++) uref[m] = U[m * ps + p0];
+      }
+      iface_upwind<UPW, 0, MX>(P, S.xi[0], S.xi[1], S.xi[2], S.xi[3], i + (long long)(N0 + 1) * j, U, pR - 1, pR,
+                               uref, sx + jj * LX + ii, NX);
+    }
+  }
+  if (!GIVEN && tid < NY) {      // TI x (TJ + 1) y interfaces
+    int ii, jj;
+    if (YM == Y_TRANSPOSED) { jj = tid % LY; ii = tid / LY; }
+    else { ii = tid % TI; jj = tid / TI; }
+    const int i = i0 + ii, j = j0 + jj;
+    if (j <= N1 && i < N0) {
+      if (MX && (UPW == UPW_LLF || UPW == UPW_RF)) {
+        const long long p0 = pidx(P, i, 0);
+#pragma unroll
+        for (int m = 0; m < 4; m++) uref[m] = U[m * ps + p0];
+      }
+      if (YM == Y_TRANSPOSED) {
+        const long long pR = (long long)(j + g) + (long long)P.W1 * (i + g);
+        iface_upwind<UPW, 1, MX>(P, S.yi[0], S.yi[1], S.yi[2], S.yi[3], j + (long long)(N1 + 1) * i, S.UT, pR - 1,
+                                 pR, uref, sy + ii * LY + jj, NY);
+      } else {
+        const long long pR = pidx(P, i, j);
+        iface_upwind<UPW, 1, MX>(P, S.yi[0], S.yi[1], S.yi[2], S.yi[3], i + (long long)N0 * j, U, pR - P.W0, pR,
+                                 uref, sy + ii * LY + jj, NY);
+      }
+    }
+  }
+  __syncthreads();
   if (tid >= TI * TJ) return;
   const int ii = tid % TI, jj = tid / TI;
   const int i = i0 + ii, j = j0 + jj;
