@@ -161,9 +161,13 @@ __global__ void __launch_bounds__(256) k_transpose_flux_y(DevParams P, const dou
 // after another with two barriers each, took 18 us of latency, and a step 95
 // us where it takes 83 with the variables in blocks of their own; where the
 // tiles fill the GPU the second reading costs more than the barriers (512^2: 33
-// against 29 us, 2048^2: 353 against 279).
-__global__ void __launch_bounds__(256) k_transpose_flux_y_parts(DevParams P, const double* __restrict__ U,
-                                                          double* __restrict__ UT, double* __restrict__ FT) {
+// against 29 us, 2048^2: 353 against 279).  R: rows of threads; up to one block
+// an SM a thread a point (R = 32), which takes the 64^2 grid's kernel from 9.8 to
+// 6.2 us and its step from 80 to 74, more blocks with four points a thread.
+template <int R>
+__global__ void __launch_bounds__(32 * R) k_transpose_flux_y_parts(DevParams P, const double* __restrict__ U,
+                                                                   double* __restrict__ UT, double* __restrict__ FT) {
+  constexpr int K = 32 / R;   // points a thread
   __shared__ double tile[4][32][33];
   const int W0 = P.W0, W1 = P.W1, parts = P.nvars - 3, part = blockIdx.x % parts;
   const long long ps = P.ps;
@@ -171,10 +175,10 @@ __global__ void __launch_bounds__(256) k_transpose_flux_y_parts(DevParams P, con
   const int tx = threadIdx.x, ty = threadIdx.y;
   if (part > 0) {
     const int m = 3 + part;
-    double x[4], r[4], v[4];
+    double x[K], r[K], v[K];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int i = i0 + tx, j = j0 + ty + 8 * k;
+    for (int k = 0; k < K; k++) {
+      const int i = i0 + tx, j = j0 + ty + R * k;
       const bool in = i < W0 && j < W1;
       const long long p = (long long)j * W0 + i;
       x[k] = in ? U[m * ps + p] : 0.0;
@@ -182,33 +186,33 @@ __global__ void __launch_bounds__(256) k_transpose_flux_y_parts(DevParams P, con
       v[k] = in ? U[2 * ps + p] : 0.0;
     }
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      tile[0][ty + 8 * k][tx] = x[k];
-      tile[1][ty + 8 * k][tx] = __dmul_rn(r[k] == 0.0 ? 0.0 : v[k] / r[k], x[k]);
+    for (int k = 0; k < K; k++) {
+      tile[0][ty + R * k][tx] = x[k];
+      tile[1][ty + R * k][tx] = __dmul_rn(r[k] == 0.0 ? 0.0 : v[k] / r[k], x[k]);
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int i = i0 + ty + 8 * k, j = j0 + tx;
+    for (int k = 0; k < K; k++) {
+      const int i = i0 + ty + R * k, j = j0 + tx;
       if (i < W0 && j < W1) {
         const long long q = (long long)i * W1 + j;
-        UT[m * ps + q] = tile[0][tx][ty + 8 * k];
-        FT[m * ps + q] = tile[1][tx][ty + 8 * k];
+        UT[m * ps + q] = tile[0][tx][ty + R * k];
+        FT[m * ps + q] = tile[1][tx][ty + R * k];
       }
     }
     return;
   }
 #pragma unroll
   for (int m = 0; m < 4; m++)
-    for (int r = ty; r < 32; r += 8) {
+    for (int r = ty; r < 32; r += R) {
       const int i = i0 + tx, j = j0 + r;
       if (i < W0 && j < W1) tile[m][r][tx] = U[m * ps + (long long)j * W0 + i];
     }
   __syncthreads();
   // point (i = i0 + r, j = j0 + tx): writes along j are coalesced
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int r = ty + 8 * k;
+  for (int k = 0; k < K; k++) {
+    const int r = ty + R * k;
     const int j = j0 + tx, i = i0 + r;
     if (i < W0 && j < W1) {
       double f[4], vn;
@@ -1023,7 +1027,10 @@ void launch_transpose_flux_y(const DevParams& P, const double* U, double* UT, do
   const unsigned tx = nblk(P.W0, 32), ty = nblk(P.W1, 32);
   const dim3 blk(32, 8);
   // up to one tile an SM the tiles' variables in blocks of their own
-  if (tx * ty <= 148 && P.nvars > 4) k_transpose_flux_y_parts<<<dim3(tx * (P.nvars - 3), ty), blk, 0, s>>>(P, U, UT, FT);
+  // (up to one such block an SM with a thread a point)
+  const dim3 grid(tx * (P.nvars - 3), ty);
+  if (P.nvars > 4 && grid.x * ty <= 148) k_transpose_flux_y_parts<32><<<grid, dim3(32, 32), 0, s>>>(P, U, UT, FT);
+  else if (P.nvars > 4 && tx * ty <= 148) k_transpose_flux_y_parts<8><<<grid, blk, 0, s>>>(P, U, UT, FT);
   else k_transpose_flux_y<<<dim3(tx, ty), blk, 0, s>>>(P, U, UT, FT);
 }
 void launch_transpose(const DevParams& P, const double* in, double* out, cudaStream_t s) {
