@@ -44,6 +44,18 @@ enum YMode { Y_STD = 0, Y_TRANSPOSED = 1, Y_GIVEN = 2 };
 // 18.4); RF's matrices in FP64 two (1201 x 777: 131.1 us, 133.3 with three).
 constexpr int stage2d_ctas(int upw, bool mx) { return mx ? 4 : upw == UPW_RF ? 2 : 3; }
 
+// Threads a CTA.  Up to one tile an SM 512: x and y interfaces by different
+// threads, the chemistry beside the viscous fluxes, a point's variables by two
+// threads -- what counts there is the length of one thread's work (64 x 64: two
+// warps a scheduler, 7 clocks an instruction).  A step, LLF with chemistry, from
+// 256 to 512 threads: 16 x 16 66 -> 55 us, 64 x 64 80 -> 69, 176 x 176 (143 tiles)
+// 124 -> 114; Roe, WENO5: 64 x 64 66 -> 56, 176 x 176 88 -> 78.  Past 148 tiles
+// the wider CTA, of which an SM holds one (at the 64 registers of two it would
+// spill), would need a second round where three of 256 threads need one.
+constexpr int WIDE = 512, NARROW = 256;
+// the variables of a point from which a wide CTA's second half works on
+constexpr int second_half(int nv) { return nv == 11 ? 5 : 2; }
+
 template <typename T>
 constexpr size_t stage2d_smem(int nv, bool given, bool visc) {
   // interface fluxes, after velocities and temperature in the same place; the
@@ -145,8 +157,9 @@ __device__ __forceinline__ void iface_upwind(const DevParams& P, const void* __r
 
 // NV: the number of variables when it is 11 (one chemistry layer) or 4 (none),
 // 0 for any other: the registers hold the point's variables group by group.
-template <int UPW, int YM, bool MX, int NV>
-__global__ void __launch_bounds__(256, stage2d_ctas(UPW, MX)) k_stage2d(DevParams P, Stage2D S) {
+// BT: WIDE (NV > 0 only) or NARROW threads.
+template <int UPW, int YM, bool MX, int NV, int BT>
+__global__ void __launch_bounds__(BT, BT == WIDE ? 1 : stage2d_ctas(UPW, MX)) k_stage2d(DevParams P, Stage2D S) {
   typedef typename std::conditional<MX, float, double>::type T;
   extern __shared__ double sfd[];
   constexpr bool GIVEN = YM == Y_GIVEN;
@@ -157,6 +170,8 @@ __global__ void __launch_bounds__(256, stage2d_ctas(UPW, MX)) k_stage2d(DevParam
   const int i0 = blockIdx.x * TI, j0 = blockIdx.y * TJ;
   const int tid = threadIdx.x;
   const bool visc = S.visc != 0;
+  // the thread's point and, in a wide CTA, its half of the point's variables
+  const int half = BT == WIDE ? tid / 256 : 0, pt = BT == WIDE ? tid % 256 : tid;
   T* sVx = (T*)sfd;                           // viscous x fluxes [3][TJ][FX]
   T* sVy = sVx + (visc ? 3 * TJ * FX : 0);    // viscous y fluxes [3][FY][TI]
   T* sx = sVy + (visc ? 3 * FY * TI : 0);     // x-interface fluxes [m][row jj][ii = 0..TI]
@@ -167,7 +182,7 @@ __global__ void __launch_bounds__(256, stage2d_ctas(UPW, MX)) k_stage2d(DevParam
   double* sT_ = (double*)sx;
   T* sQ = (T*)(sT_ + QX * QY);
   if (visc) {
-    for (int e = tid; e < QX * QY; e += 256) {
+    for (int e = tid; e < QX * QY; e += BT) {
       const int a = e % QX, b = e / QX;
       const int i = i0 - 1 + a, j = j0 - 1 + b;
       double uu = 0.0, vv = 0.0, TT = 0.0;
@@ -221,8 +236,25 @@ __global__ void __launch_bounds__(256, stage2d_ctas(UPW, MX)) k_stage2d(DevParam
         }
       }
     }
-    __syncthreads();
   }
+  // wide: the chemistry source of point pt by the second half, beside the viscous
+  // fluxes; its heat release to the first half
+  __shared__ double sH[BT == WIDE && NV == 11 ? TI * TJ : 1];
+  T src[5], Q = T(0);
+  auto chemistry = [&](int i, int j) {
+    const long long p = pidx(P, i, j);
+    const double t = *S.tdev + S.cstage * P.dt;
+    const T n_hnu = chem_hnu0<T>(P, pulse_factor(P, t), S.imap[p]);
+    if (S.hnu) S.hnu[p] = (double)n_hnu;
+    const double* s = U + 4 * ps + p;
+    chem_layer<T>(P, n_hnu, (T)s[0], (T)s[ps], (T)s[2 * ps], (T)s[3 * ps], (T)s[4 * ps], (T)s[5 * ps],
+                  (T)s[6 * ps], src, Q);
+  };
+  if (BT == WIDE && NV == 11 && S.chem && half && pt < TI * TJ && i0 + pt % TI < N0 && j0 + pt / TI < N1) {
+    chemistry(i0 + pt % TI, j0 + pt / TI);
+    sH[pt] = (double)Q;
+  }
+  if (visc) __syncthreads();
   double uref[4];
   if (tid < NX) {                // (TI + 1) x TJ x interfaces
     const int ii = tid % LX, jj = tid / LX;
@@ -238,10 +270,11 @@ __global__ void __launch_bounds__(256, stage2d_ctas(UPW, MX)) k_stage2d(DevParam
                                uref, sx + jj * LX + ii, NX);
     }
   }
-  if (!GIVEN && tid < NY) {      // TI x (TJ + 1) y interfaces
+  const int ty = BT == WIDE ? tid - 256 : tid;
+  if (!GIVEN && ty >= 0 && ty < NY) {   // TI x (TJ + 1) y interfaces
     int ii, jj;
-    if (YM == Y_TRANSPOSED) { jj = tid % LY; ii = tid / LY; }
-    else { ii = tid % TI; jj = tid / TI; }
+    if (YM == Y_TRANSPOSED) { jj = ty % LY; ii = ty / LY; }
+    else { ii = ty % TI; jj = ty / TI; }
     const int i = i0 + ii, j = j0 + jj;
     if (j <= N1 && i < N0) {
       if (MX && (UPW == UPW_LLF || UPW == UPW_RF)) {
@@ -261,8 +294,8 @@ __global__ void __launch_bounds__(256, stage2d_ctas(UPW, MX)) k_stage2d(DevParam
     }
   }
   __syncthreads();
-  if (tid >= TI * TJ) return;
-  const int ii = tid % TI, jj = tid / TI;
+  if (pt >= TI * TJ) return;
+  const int ii = pt % TI, jj = pt / TI;
   const int i = i0 + ii, j = j0 + jj;
   if (i >= N0 || j >= N1) return;
   const long long p = pidx(P, i, j);
@@ -286,15 +319,8 @@ __global__ void __launch_bounds__(256, stage2d_ctas(UPW, MX)) k_stage2d(DevParam
     const T* vy = sVy + (m - 1) * FY * TI + jj * TI + ii;
     return (double)fma_rn(dxi, vx[1] - vx[0], mul_rn(dyi, vy[TI] - vy[0]));
   };
-  T src[5], Q = T(0);
-  if (NV == 11 && S.chem) {
-    const double t = *S.tdev + S.cstage * P.dt;
-    const T n_hnu = chem_hnu0<T>(P, pulse_factor(P, t), S.imap[p]);
-    if (S.hnu) S.hnu[p] = (double)n_hnu;
-    const double* s = U + 4 * ps + p;
-    chem_layer<T>(P, n_hnu, (T)s[0], (T)s[ps], (T)s[2 * ps], (T)s[3 * ps], (T)s[4 * ps], (T)s[5 * ps],
-                  (T)s[6 * ps], src, Q);
-  }
+  if (BT == NARROW && NV == 11 && S.chem) chemistry(i, j);
+  if (BT == WIDE && NV == 11 && S.chem && !half) Q = (T)sH[pt];
   // the stage derivative of variable m
   auto deriv = [&](int m) -> double {
     double k = S.neg ? -hyp(m) : hyp(m);
@@ -309,33 +335,45 @@ __global__ void __launch_bounds__(256, stage2d_ctas(UPW, MX)) k_stage2d(DevParam
     // groups of variables: the loads of the earlier stages' part of the
     // combination in flight together, then the derivatives, then the stores
     constexpr int NG = 4;
-#pragma unroll
-    for (int m0 = 0; m0 < NV; m0 += NG) {
+    auto group = [&](int m0, int end) {
       double xa[NG];
       if (S.dst) {
 #pragma unroll
         for (int w = 0; w < NG; w++)
-          if (m0 + w < NV) xa[w] = S.u[(m0 + w) * ps + p];
+          if (m0 + w < end) xa[w] = S.u[(m0 + w) * ps + p];
         for (int q = 0; q < S.nprev; q++) {
           const double a = S.a[q];
           const double* d = S.d[q] + p;
           double t[NG];
 #pragma unroll
           for (int w = 0; w < NG; w++)
-            if (m0 + w < NV) t[w] = d[(m0 + w) * ps];
+            if (m0 + w < end) t[w] = d[(m0 + w) * ps];
 #pragma unroll
           for (int w = 0; w < NG; w++)
-            if (m0 + w < NV) xa[w] = fma_rn(a, t[w], xa[w]);
+            if (m0 + w < end) xa[w] = fma_rn(a, t[w], xa[w]);
         }
       }
 #pragma unroll
       for (int w = 0; w < NG; w++)
-        if (m0 + w < NV) {
+        if (m0 + w < end) {
           const int m = m0 + w;
           const double k = deriv(m);
           if (S.k) S.k[m * ps + p] = k;
           if (S.dst) S.dst[m * ps + p] = fma_rn(S.as, k, xa[w]);
         }
+    };
+    if (BT == WIDE) {
+      constexpr int MH = second_half(NV);
+      if (half) {
+#pragma unroll
+        for (int m0 = MH; m0 < NV; m0 += NG) group(m0, NV);
+      } else {
+#pragma unroll
+        for (int m0 = 0; m0 < MH; m0 += NG) group(m0, MH);
+      }
+    } else {
+#pragma unroll
+      for (int m0 = 0; m0 < NV; m0 += NG) group(m0, NV);
     }
   } else {
     // any number of layers: the derivative through memory
@@ -399,12 +437,19 @@ __global__ void __launch_bounds__(256, UPW == UPW_RF && !MX ? 2 : 3) k_slab_upwi
     out[(long long)m * n1 * N0] = mul_rn(dyi, sy[m * NY + ii * LY + jj + 1] - sy[m * NY + ii * LY + jj]);
 }
 
+template <int UPW, int YM, bool MX, int NV, int BT>
+void stage2d_bt(const DevParams& P, const Stage2D& S, dim3 grid, cudaStream_t s) {
+  typedef typename std::conditional<MX, float, double>::type T;
+  raise_smem_limit<k_stage2d<UPW, YM, MX, NV, BT>>(200 * 1024);
+  k_stage2d<UPW, YM, MX, NV, BT><<<grid, BT, stage2d_smem<T>(P.nvars, YM == Y_GIVEN, S.visc), s>>>(P, S);
+}
 template <int UPW, int YM, bool MX, int NV>
 void stage2d_nv(const DevParams& P, const Stage2D& S, cudaStream_t s) {
-  typedef typename std::conditional<MX, float, double>::type T;
-  raise_smem_limit<k_stage2d<UPW, YM, MX, NV>>(200 * 1024);
   const dim3 grid((P.N0 + TI - 1) / TI, (P.N1 + TJ - 1) / TJ);
-  k_stage2d<UPW, YM, MX, NV><<<grid, 256, stage2d_smem<T>(P.nvars, YM == Y_GIVEN, S.visc), s>>>(P, S);
+  if constexpr (NV > 0 && YM != Y_GIVEN) {
+    if (grid.x * grid.y <= 148) return stage2d_bt<UPW, YM, MX, NV, WIDE>(P, S, grid, s);
+  }
+  stage2d_bt<UPW, YM, MX, NV, NARROW>(P, S, grid, s);
 }
 template <int UPW, int YM, bool MX>
 void stage2d_upw(const DevParams& P, const Stage2D& S, cudaStream_t s) {
