@@ -13,7 +13,7 @@
 // Separate kernels for the upwinding, the viscous terms and source, and the
 // combination read and wrote the derivative three times over: at 2048^2 with 11
 // variables 0.53 + 0.31 ms and 0.2 ms of combination a stage, where this takes
-// 0.68 ms with the combination; a step of the 512^2 run went from 640 to 574 us,
+// 0.67 ms with the combination; a step of the 512^2 run went from 640 to 574 us,
 // one of 300 x 217 points from 198 to 161 us.  Three CTAs an SM (80 registers)
 // hide the loads; the 16 x 15 tile of the upwinding alone would put 16 points of
 // the viscous fluxes in a second round.
@@ -130,26 +130,28 @@ __device__ __forceinline__ void iface_upwind(const DevParams& P, const void* __r
   }
 #pragma unroll
   for (int m = 0; m < NF; m++) so[m * stride] = fi[m];
-  // passive variables four at a time, their loads in flight together
+  // passive variables seven at a time (a chemistry layer), their loads in flight
+  // together: 0.666 ms at 2048^2 where four at a time take 0.697
   const int nv = P.nvars;
-  for (int m = NF; m < nv; m += 4) {
-    T du[4], sf[4];
+  constexpr int G = 7;
+  for (int m = NF; m < nv; m += G) {
+    T du[G], sf[G];
     if (P.pack_sp) {
 #pragma unroll
-      for (int k = 0; k < 4; k++)
+      for (int k = 0; k < G; k++)
         if (m + k < nv) { du[k] = uL[(m + k) * is]; sf[k] = fL[(m + k) * is]; }
 #pragma unroll
-      for (int k = 0; k < 4; k++)
+      for (int k = 0; k < G; k++)
         if (m + k < nv) so[(m + k) * stride] = upwind_species_packed(spm, spa, du[k], sf[k]);
     } else {
-      T l[4], r[4];
+      T l[G], r[G];
 #pragma unroll
-      for (int k = 0; k < 4; k++)
+      for (int k = 0; k < G; k++)
         if (m + k < nv) {
           l[k] = uL[(m + k) * is]; r[k] = uR[(m + k) * is]; du[k] = fL[(m + k) * is]; sf[k] = fR[(m + k) * is];
         }
 #pragma unroll
-      for (int k = 0; k < 4; k++)
+      for (int k = 0; k < G; k++)
         if (m + k < nv) so[(m + k) * stride] = upwind_species(spm, spa, l[k], r[k], du[k], sf[k]);
     }
   }
