@@ -132,8 +132,9 @@ int piafs_gpu_synchronize(piafs_gpu_sim* sim);
  * evaluations.  ms[k] receives the mean duration of phase k; phases are, per
  * direction d = 0..ndims-1, [2d] flux (with the transpose of a transposed
  * y pass), [2d+1] interface reconstruction (WENO5 or the CRWENO5 line
- * solve), then [2 ndims] upwinding + divergence of all directions and
- * [2 ndims + 1] viscous + source.  nphases (in/out) is the capacity / count. */
+ * solve), then [2 ndims] upwinding + divergence of all directions (in 2D with
+ * second-order viscous terms these and the source too, one kernel) and
+ * [2 ndims + 1] viscous + source where they are apart, and the sponge zones.  nphases (in/out) is the capacity / count. */
 int piafs_gpu_profile_rhs(piafs_gpu_sim* sim, int reps, double* ms, int* nphases);
 
 /* Photon density of the last RK stage evaluated (the reference's
