@@ -506,8 +506,46 @@ __global__ void k_weno5(DevParams P, const double* __restrict__ U, const double*
 // component one.  One thread per interface.  (The reference takes the
 // average of the cells in the order of each bias; it is the same state to
 // rounding, and one average serves both biases here.)
+// The characteristic fields of the average of two cells: matrices, or for 2D
+// Navier-Stokes the closed form (NsFields).  The kernel is bound by FP64 latency
+// at the threads an SM holds: the two 4 x 4 matrices kept 128 registers (96 and 99
+// us a direction at 1201 x 777); in closed form 74 and 78, at five blocks an SM (102
+// registers) 68 and 73, at six 69 and 74.
+template <int MODEL>
+struct CharFields {
+  static constexpr int NF = Flow<MODEL>::NF;
+  double L[4][4], R[4][4];
+  __device__ __forceinline__ void set(const double* cl, const double* cr, double gamma, int dir) {
+    double ua[4];
+    Flow<MODEL>::roe_avg(cl, cr, gamma, ua);
+    Flow<MODEL>::eigvec(ua, gamma, dir, L, R);
+  }
+  __device__ __forceinline__ void left(const double* x, int, double* w) const {
+#pragma unroll
+    for (int v = 0; v < NF; v++) {
+      double acc = 0.0;
+#pragma unroll
+      for (int k = 0; k < NF; k++) acc += L[v][k] * x[k];
+      w[v] = acc;
+    }
+  }
+  __device__ __forceinline__ void right(const double* w, int, double* f) const {
+#pragma unroll
+    for (int k = 0; k < NF; k++) {
+#pragma unroll
+      for (int v = 0; v < NF; v++) f[k] += R[k][v] * w[v];
+    }
+  }
+};
+template <>
+struct CharFields<NS2D> : NsFields<double> {
+  __device__ __forceinline__ void set(const double* cl, const double* cr, double gamma, int dir) {
+    double vnL, cL, vnR, cR;
+    ns2d_fields<double>(cl, cr, gamma, dir, *this, vnL, cL, vnR, cR);
+  }
+};
 template <int MODEL, int DIR>
-__global__ void k_weno5_char(DevParams P, const double* __restrict__ U, const double* __restrict__ F,
+__global__ void __launch_bounds__(128, 5) k_weno5_char(DevParams P, const double* __restrict__ U, const double* __restrict__ F,
                              double* __restrict__ uL, double* __restrict__ uR, double* __restrict__ fL,
                              double* __restrict__ fR) {
   constexpr int NF = Flow<MODEL>::NF;
@@ -519,40 +557,37 @@ __global__ void k_weno5_char(DevParams P, const double* __restrict__ U, const do
   const long long st = DIR == 0 ? 1 : P.W0;
   const long long c0 = cell_of<DIR>(P, i, l);    // cell i (right of the interface)
   const long long ps = P.ps;
-  double cl[4], cr[4], ua[4], L[4][4], R[4][4];
+  double cl[4], cr[4];
 #pragma unroll
   for (int m = 0; m < NF; m++) { cl[m] = U[m * ps + c0 - st]; cr[m] = U[m * ps + c0]; }
-  Flow<MODEL>::roe_avg(cl, cr, P.gamma, ua);
-  Flow<MODEL>::eigvec(ua, P.gamma, DIR, L, R);
+  CharFields<MODEL> C;
+  C.set(cl, cr, P.gamma, DIR);
 #pragma unroll
   for (int fld = 0; fld < 2; fld++) {
     const double* src = fld ? F : U;
-    double w[NF][6];                              // characteristic values, cells i-3 .. i+2
+    double w[6][4];                               // characteristic values, cells i-3 .. i+2
 #pragma unroll
     for (int r = 0; r < 6; r++) {
       double cv[4];
 #pragma unroll
       for (int m = 0; m < NF; m++) cv[m] = src[m * ps + c0 + (r - 3) * st];
-#pragma unroll
-      for (int v = 0; v < NF; v++) {
-        double acc = 0.0;
-#pragma unroll
-        for (int k = 0; k < NF; k++) acc += L[v][k] * cv[k];
-        w[v][r] = acc;
-      }
+      C.left(cv, DIR, w[r]);
     }
     double vl[4], vr[4];
 #pragma unroll
-    for (int v = 0; v < NF; v++) weno5_pair(P, w[v], vl[v], vr[v]);
+    for (int v = 0; v < NF; v++) {
+      const double c[6] = {w[0][v], w[1][v], w[2][v], w[3][v], w[4][v], w[5][v]};
+      weno5_pair(P, c, vl[v], vr[v]);
+    }
     double* oL = fld ? fL : uL;
     double* oR = fld ? fR : uR;
+    double sl[4] = {0.0, 0.0, 0.0, 0.0}, sr[4] = {0.0, 0.0, 0.0, 0.0};
+    C.right(vl, DIR, sl);
+    C.right(vr, DIR, sr);
 #pragma unroll
     for (int k = 0; k < NF; k++) {
-      double sl = 0.0, sr = 0.0;
-#pragma unroll
-      for (int v = 0; v < NF; v++) { sl += R[k][v] * vl[v]; sr += R[k][v] * vr[v]; }
-      oL[k * P.pis + q] = sl;
-      oR[k * P.pis + q] = sr;
+      oL[k * P.pis + q] = sl[k];
+      oR[k * P.pis + q] = sr[k];
     }
   }
   for (int m = NF; m < P.nvars; m++) {
