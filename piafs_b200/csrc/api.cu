@@ -473,8 +473,11 @@ int piafs::create_sim(Deck&& deck, int precision, piafs_gpu_sim** out) {
   }
   s->U[0] = s->u;
   // one-stage schemes advance u itself, which other tiles still read as the
-  // stage's state: their combination stays a kernel of its own
-  s->fuse_rk = P.ndims == 2 && !visc4(P) && s->sponges.empty() && d.nstages > 1;
+  // stage's state: their combination stays a kernel of its own.  So does that
+  // of a grid narrower than its ghost layers: its boundary fill reads ghosts of
+  // the face across before it writes them, and they must be this step's of u,
+  // which only the combination over all points carries into a stage's state
+  s->fuse_rk = P.ndims == 2 && !visc4(P) && s->sponges.empty() && d.nstages > 1 && !narrow_grid(P);
   setup_run1d(s);
   // initial solution; restart time waqt = restart_iter * dt (TimeInitialize.c:51)
   int rr = piafs_gpu_set_state(s, d.u0.data(), d.restart_iter * d.dt);

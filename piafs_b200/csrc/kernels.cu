@@ -1099,7 +1099,7 @@ DevParams transposed_params(const DevParams& P) {
 // each zone is a launch.  Returns the number of launches (u null: counted
 // only).
 int launch_bc(const DevParams& P, double* u, const Zone* z, int nz, cudaStream_t s) {
-  const bool narrow = P.N0 < P.ghosts || (P.ndims == 2 && P.N1 < P.ghosts);
+  const bool narrow = narrow_grid(P);
   int launches = 0;
   auto overlap = [](const Zone& a, const Zone& b) {
     for (int d = 0; d < 2; d++)

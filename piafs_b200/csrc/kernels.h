@@ -148,6 +148,9 @@ void launch_soa_to_interior(const DevParams& P, const double* soa, double* out, 
 void launch_interior_to_soa(const DevParams& P, const double* in, double* soa, cudaStream_t s);
 void launch_iface_aos_to_soa(const double* aos, double* soa, long long ni, int nv, long long pis, cudaStream_t s);
 void launch_iface_soa_to_aos(const double* soa, double* aos, long long ni, int nv, long long pis, cudaStream_t s);
+// whether the grid is narrower than the ghost layers: a zone's source can then
+// itself be a ghost, of the face across
+inline bool narrow_grid(const DevParams& P) { return P.N0 < P.ghosts || (P.ndims == 2 && P.N1 < P.ghosts); }
 // the deck's boundary zones applied to the ghosts of u, in the deck's order;
 // returns the number of launches (u null: counted, not launched)
 int launch_bc(const DevParams& P, double* u, const Zone* z, int nz, cudaStream_t s);
