@@ -302,8 +302,17 @@ static void setup_run1d(piafs_gpu_sim* s) {
 static int run_steps(piafs_gpu_sim* s, int nsteps, bool norm_last) {
   int k0 = 0;
   if (s->run1d_ctas > 0) {
-    k0 = norm_last ? nsteps - 1 : nsteps;   // a step with the norm: kernel by kernel
-    if (int r = enqueue_run1d(s, k0)) return r;
+    // a step with the norm is one of the same steps, its start kept: the state
+    // must not depend on whether the norm is asked for
+    k0 = nsteps;
+    if (int r = enqueue_run1d(s, norm_last ? nsteps - 1 : nsteps)) return r;
+    if (norm_last) {
+      CK(cudaMemcpyAsync(s->scratch, s->u, (size_t)s->P.nvars * s->P.ps * sizeof(double), cudaMemcpyDeviceToDevice,
+                         s->stream));
+      if (int r = enqueue_run1d(s, 1)) return r;
+      CK(cudaMemsetAsync(s->norm_acc, 0, sizeof(double), s->stream));
+      launch_norm(s->P, s->scratch, s->u, s->norm_acc, s->stream);
+    }
   }
   for (int k = k0; k < nsteps; k++) {
     const bool with_norm = norm_last && (k == nsteps - 1);

@@ -393,6 +393,22 @@ __global__ void k_update2(DevParams P, double* __restrict__ u, const double* __r
   }
 }
 
+// The same sum from the states before and after a step, for steps that another
+// kernel completes without it (1D lines run in one launch): a thread per
+// interior value.
+__global__ void __launch_bounds__(256) k_norm(DevParams P, const double* __restrict__ before,
+                                              const double* __restrict__ after, double* __restrict__ acc) {
+  const long long n = (long long)P.N0 * P.N1, e = blockIdx.x * 256LL + threadIdx.x;
+  double sq = 0.0;
+  if (e < n * P.nvars) {
+    const long long q = e % n, p = e / n * P.ps + pidx(P, (int)(q % P.N0), (int)(q / P.N0));
+    const double d = before[p] - after[p];
+    sq = d * d;
+  }
+  for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(acc, sq);
+}
+
 // max local CFL over interior points (NavierStokes2DComputeCFL.c:19-56,
 // Euler1DComputeCFL.c).  Non-negative doubles order like their bit patterns.
 __global__ void k_cfl(DevParams P, const double* __restrict__ u, const double* __restrict__ dxinv,
@@ -1165,6 +1181,9 @@ void launch_update(const DevParams& P, double* u, const double* const* d, const 
   k_update<<<nblk(n, 256), 256, 0, s>>>(P, u, d[0], b[0], ns > 1 ? d[1] : nullptr, ns > 1 ? b[1] : 0.0,
                                          ns > 2 ? d[2] : nullptr, ns > 2 ? b[2] : 0.0, ns > 3 ? d[3] : nullptr,
                                          ns > 3 ? b[3] : 0.0, ns, norm_acc);
+}
+void launch_norm(const DevParams& P, const double* before, const double* after, double* acc, cudaStream_t s) {
+  k_norm<<<nblk((long long)P.N0 * P.N1 * P.nvars, 256), 256, 0, s>>>(P, before, after, acc);
 }
 void launch_cfl(const DevParams& P, const double* u, const double* dxinv, unsigned long long* out, cudaStream_t s) {
   k_cfl<<<nblk((long long)P.N0 * P.N1, 256), 256, 0, s>>>(P, u, dxinv, out);

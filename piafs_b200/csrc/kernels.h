@@ -165,6 +165,8 @@ void launch_stage(long long n, double* Us, const double* u, const double* const*
                   cudaStream_t s);
 void launch_update(const DevParams& P, double* u, const double* const* d, const double* b, int ns, double* norm_acc,
                    cudaStream_t s);
+// the sum of squares of a step's change over the interior points, added to acc
+void launch_norm(const DevParams& P, const double* before, const double* after, double* acc, cudaStream_t s);
 void launch_cfl(const DevParams& P, const double* u, const double* dxinv, unsigned long long* out, cudaStream_t s);
 void launch_flux(const DevParams& P, const double* U, double* F, int dir, cudaStream_t s);
 // WENO5 interface values; doubles, or floats relative to each line's first

@@ -80,3 +80,46 @@ def test_grids_narrower_than_their_ghosts(tmp_path, rk, zones, N, NY):
     cases.ns2d_channel(d, zones, N=N, NY=NY, n_iter=3, dt=2e-3, par="2", time_scheme_type=rk, flow=(0.3, 0.2),
                        bump=0.2, bump_at=(0.4, 0.3), bump_radius=0.4)
     check(d, 2e-3, rk)
+
+
+LINE_ENDS = {"periodic": None,
+             "walls": [Z("slip-wall", 0, 1, [0.0, 0.0], [0.1]), Z("slip-wall", 0, -1, [0.0, 0.0], [0.0])],
+             "fixed": [Z("dirichlet", 0, 1, [0.0, 0.0], values=[1.0, 1.0, 3.0]), Z("extrapolate", 0, -1, [0.0, 0.0])]}
+
+
+@pytest.mark.parametrize("scheme,upw,weno,N,rk,ends", [
+    ("weno5", "roe", None, 16, "33", "periodic"), ("weno5", "roe", None, 129, "44", "walls"),
+    ("weno5", "llf-char", {"yc": 1}, 257, "ssprk3", "fixed"), ("weno5", "rf-char", {"mapped": 1}, 1009, "22", "walls"),
+    ("weno5", "rusanov", {"borges": 1}, 8192, "ssprk3", "periodic"), ("upw5", "roe", None, 300, "44", "fixed"),
+    ("crweno5", "roe", None, 17, "44", "walls"), ("crweno5", "llf-char", {"yc": 1}, 259, "33", "fixed"),
+    ("crweno5", "rusanov", None, 700, "ssprk3", "walls"), ("crweno5", "rf-char", {"mapped": 1}, 4097, "22", "periodic"),
+    ("crweno5", "roe", {"borges": 1}, 6001, "ssprk3", "fixed")])
+def test_lines(tmp_path, scheme, upw, weno, N, rk, ends):
+    """1D lines whose whole steps are one launch."""
+    d = str(tmp_path / "l")
+    cases.euler1d_density_wave(d, N=N, n_iter=3, dt=0.1 / N, scheme=scheme, upwinding=upw, weno=weno,
+                               time_scheme_type=rk, zones=LINE_ENDS[ends])
+    check(d, 0.1 / N, rk)
+
+
+@pytest.mark.parametrize("rk", ["22", "33", "44", "ssprk3"])
+@pytest.mark.parametrize("layers", [0, 1, 2])
+@pytest.mark.parametrize("N,NY,scheme,upw", [(33, 29, "crweno5", "llf-char"), (200, 230, "weno5", "roe")])
+def test_grids(tmp_path, N, NY, scheme, upw, layers, rk):
+    """The combination formed by the kernel that ends a stage, on either side of
+    148 tiles of 16 x 14, for 4, 11 and 18 variables: what a wall leaves of the
+    passive variables' ghosts, corners included, is u's in every stage.  There
+    every ghost gets a value of its own."""
+    d = str(tmp_path / "g")
+    cases.ns2d_photochem_beam(d, N=N, NY=NY, n_iter=3, dt=2e-4, scheme=scheme, upwinding=upw, time_scheme_type=rk,
+                              chemistry=layers > 0, layers=max(layers, 1), noise=1e-2, flow=(0.2, 0.1), zones=walls(),
+                              extra_chem={"z_mm": 1.3} if layers == 2 else None)
+    with Simulation(d) as sim:
+        u = sim.state().reshape(NY + 6, N + 6, -1)
+        sim.ApplyBoundaryConditions(t := torch.from_numpy(u).cuda().contiguous())
+        u = t.cpu().numpy()
+    rng = np.random.default_rng(N)
+    for a, b in ((slice(0, 3), slice(None)), (slice(NY + 3, None), slice(None)), (slice(None), slice(0, 3)),
+                 (slice(None), slice(N + 3, None))):
+        u[a, b] = 1.0 + 0.1 * rng.uniform(size=u[a, b].shape)
+    check(d, 2e-4, rk, u.reshape(-1))
