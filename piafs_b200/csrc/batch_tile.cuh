@@ -261,12 +261,11 @@ __device__ __forceinline__ void rk_point(const BMember& M, const BState& Sd, int
 // [nv][TY][HX] + [nv][HY][TX].  A per-tile constant is constant along every
 // grid line of the tile, so reconstruction and upwinding are unchanged by it
 // and the divergence cancels it.
-template <int TX, int TY, bool MX>
-struct Tile2D {
+// PITCH: of a row of TX + 6 cells (tile_pitch).
+template <int TX, int TY, bool MX, int PITCH>
+struct Tile2DAt {
   typedef typename std::conditional<MX, float, double>::type T;
-  // HX: the pitch of a row of TX + 6 cells, odd so that threads on different
-  // rows read different banks
-  static constexpr int HX = (TX + 6) | 1, HY = TY + 6;
+  static constexpr int HX = PITCH, HY = TY + 6;
   static constexpr int NXI = TY * (TX + 1), NYI = TX * (TY + 1), NI = NXI + NYI;
   static constexpr int NCX = TY * HX, NCY = TX * HY;            // stencil cells per direction
   // strips of at most nine consecutive interfaces of a line, one thread's work
@@ -296,7 +295,24 @@ struct Tile2D {
   __host__ __device__ static constexpr long long smem(int nv) {
     return su_bytes(nv) + fx_bytes(nv) + fy_bytes(nv) + work(nv);
   }
+  // the most layers of seven species (at most four: 32 variables) whose tile
+  // fits the 227 KB a CTA can have
+  static constexpr int layers() {
+    int k = 4;
+    while (k > 0 && smem(4 + 7 * k) > 227 * 1024) k--;
+    return k;
+  }
 };
+// Odd, so that threads on different rows read different banks, except where
+// the padding would cost members their place (FP64 32 x 4 and mixed 8 x 16: four
+// layers fit at the plain pitch only).
+template <int TX, int TY, bool MX>
+constexpr int tile_pitch() {
+  constexpr int plain = TX + 6, odd = plain | 1;
+  return Tile2DAt<TX, TY, MX, odd>::layers() < Tile2DAt<TX, TY, MX, plain>::layers() ? plain : odd;
+}
+template <int TX, int TY, bool MX>
+struct Tile2D : Tile2DAt<TX, TY, MX, tile_pitch<TX, TY, MX>()> {};
 
 // ------------------------------------------------------------- 1D tile
 // A 1D tile has T1 points, one per thread.  Shared memory (bytes): sU and
