@@ -71,8 +71,12 @@ constexpr size_t stage2d_smem(int nv, bool given, bool visc) {
 // deviation form and stored relative to the line's flux reference.  The
 // schemes other than RF need only uL - uR and fL + fR besides the states of
 // the Roe average (LLF: the interface states), and take them as they are
-// packed by the reconstruction (P.pack_sp) or form them here.
-template <int UPW, int DIR, bool MX>
+// packed by the reconstruction (P.pack_sp) or form them here.  NV: the number of
+// variables, or 0 for P.nvars; where it is 4 the loop over the passive variables
+// must not be there at all -- room for its loads, never issued, spilled 350 to 370
+// bytes a thread (132 to 136 in mixed precision with a transposed y pass), which
+// cost 0.3 to 1 % of a step at 1201 x 777 (WENO5, Rusanov 668 -> 663 us).
+template <int UPW, int DIR, bool MX, int NV>
 __device__ __forceinline__ void iface_upwind(const DevParams& P, const void* __restrict__ uLv,
                                              const void* __restrict__ uRv, const void* __restrict__ fLv,
                                              const void* __restrict__ fRv, long long q,
@@ -132,7 +136,7 @@ __device__ __forceinline__ void iface_upwind(const DevParams& P, const void* __r
   for (int m = 0; m < NF; m++) so[m * stride] = fi[m];
   // passive variables seven at a time (a chemistry layer), their loads in flight
   // together: 0.666 ms at 2048^2 where four at a time take 0.697
-  const int nv = P.nvars;
+  const int nv = NV ? NV : P.nvars;
   constexpr int G = 7;
   for (int m = NF; m < nv; m += G) {
     T du[G], sf[G];
@@ -268,7 +272,7 @@ __global__ void __launch_bounds__(BT, BT == WIDE ? 1 : stage2d_ctas(UPW, MX)) k_
 #pragma unroll
         for (int m = 0; m < 4; m++) uref[m] = U[m * ps + p0];
       }
-      iface_upwind<UPW, 0, MX>(P, S.xi[0], S.xi[1], S.xi[2], S.xi[3], i + (long long)(N0 + 1) * j, U, pR - 1, pR,
+      iface_upwind<UPW, 0, MX, NV>(P, S.xi[0], S.xi[1], S.xi[2], S.xi[3], i + (long long)(N0 + 1) * j, U, pR - 1, pR,
                                uref, sx + jj * LX + ii, NX);
     }
   }
@@ -286,11 +290,11 @@ __global__ void __launch_bounds__(BT, BT == WIDE ? 1 : stage2d_ctas(UPW, MX)) k_
       }
       if (YM == Y_TRANSPOSED) {
         const long long pR = (long long)(j + g) + (long long)P.W1 * (i + g);
-        iface_upwind<UPW, 1, MX>(P, S.yi[0], S.yi[1], S.yi[2], S.yi[3], j + (long long)(N1 + 1) * i, S.UT, pR - 1,
+        iface_upwind<UPW, 1, MX, NV>(P, S.yi[0], S.yi[1], S.yi[2], S.yi[3], j + (long long)(N1 + 1) * i, S.UT, pR - 1,
                                  pR, uref, sy + ii * LY + jj, NY);
       } else {
         const long long pR = pidx(P, i, j);
-        iface_upwind<UPW, 1, MX>(P, S.yi[0], S.yi[1], S.yi[2], S.yi[3], i + (long long)N0 * j, U, pR - P.W0, pR,
+        iface_upwind<UPW, 1, MX, NV>(P, S.yi[0], S.yi[1], S.yi[2], S.yi[3], i + (long long)N0 * j, U, pR - P.W0, pR,
                                  uref, sy + ii * LY + jj, NY);
       }
     }
@@ -423,7 +427,7 @@ __global__ void __launch_bounds__(256, UPW == UPW_RF && !MX ? 2 : 3) k_slab_upwi
         for (int m = 0; m < 4; m++) uref[m] = UT[m * P.ps + g + line];
       }
       const long long pR = (long long)(j + g) + line;
-      iface_upwind<UPW, 1, MX>(P, yuL, yuR, yfL, yfR, j + (long long)(N1 + 1) * i, UT, pR - 1, pR, uref,
+      iface_upwind<UPW, 1, MX, 0>(P, yuL, yuR, yfL, yfR, j + (long long)(N1 + 1) * i, UT, pR - 1, pR, uref,
                                sy + ii * LY + jj, NY);
     }
   }
