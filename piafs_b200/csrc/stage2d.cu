@@ -44,6 +44,15 @@ enum YMode { Y_STD = 0, Y_TRANSPOSED = 1, Y_GIVEN = 2 };
 // 18.4); RF's matrices in FP64 two (1201 x 777: 131.1 us, 133.3 with three).
 constexpr int stage2d_ctas(int upw, bool mx) { return mx ? 4 : upw == UPW_RF ? 2 : 3; }
 
+// The grid of tiles: rows of tiles in y and, past the 65535 a launch takes there,
+// in z (grids of more than 917,490 rows of points).  Tiles that this rounds up to
+// beyond the last row have no interface or point inside the grid.
+dim3 tile_grid(const DevParams& P) {
+  const int tx = (P.N0 + TI - 1) / TI, ty = (P.N1 + TJ - 1) / TJ, nz = (ty + 65534) / 65535;
+  return dim3(tx, (ty + nz - 1) / nz, nz);
+}
+__device__ __forceinline__ int tile_row() { return blockIdx.y + blockIdx.z * gridDim.y; }
+
 // Threads a CTA.  Up to one tile an SM 512: x and y interfaces by different
 // threads, the chemistry beside the viscous fluxes, a point's variables by two
 // threads -- what counts there is the length of one thread's work (64 x 64: two
@@ -173,7 +182,7 @@ __global__ void __launch_bounds__(BT, BT == WIDE ? 1 : stage2d_ctas(UPW, MX)) k_
   const int N0 = P.N0, N1 = P.N1, g = P.ghosts;
   const long long ps = P.ps;
   const double* __restrict__ U = S.U;
-  const int i0 = blockIdx.x * TI, j0 = blockIdx.y * TJ;
+  const int i0 = blockIdx.x * TI, j0 = tile_row() * TJ;
   const int tid = threadIdx.x;
   const bool visc = S.visc != 0;
   // the thread's point and, in a wide CTA, its half of the point's variables
@@ -414,7 +423,7 @@ __global__ void __launch_bounds__(256, UPW == UPW_RF && !MX ? 2 : 3) k_slab_upwi
   extern __shared__ double sfd[];
   T* sy = (T*)sfd;
   const int nvars = P.nvars, N0 = P.N0, N1 = P.N1, g = P.ghosts;
-  const int i0 = blockIdx.x * TI, j0 = blockIdx.y * TJ;
+  const int i0 = blockIdx.x * TI, j0 = tile_row() * TJ;
   const int tid = threadIdx.x;
   double uref[4];
   if (tid < NY) {
@@ -451,9 +460,9 @@ void stage2d_bt(const DevParams& P, const Stage2D& S, dim3 grid, cudaStream_t s)
 }
 template <int UPW, int YM, bool MX, int NV>
 void stage2d_nv(const DevParams& P, const Stage2D& S, cudaStream_t s) {
-  const dim3 grid((P.N0 + TI - 1) / TI, (P.N1 + TJ - 1) / TJ);
+  const dim3 grid = tile_grid(P);
   if constexpr (NV > 0 && YM != Y_GIVEN) {
-    if (grid.x * grid.y <= 148) return stage2d_bt<UPW, YM, MX, NV, WIDE>(P, S, grid, s);
+    if (grid.x * grid.y * grid.z <= 148) return stage2d_bt<UPW, YM, MX, NV, WIDE>(P, S, grid, s);
   }
   stage2d_bt<UPW, YM, MX, NV, NARROW>(P, S, grid, s);
 }
@@ -483,7 +492,7 @@ template <int UPW, bool MX>
 void slab_upwind_y_u(const DevParams& P, const double* UT, const void* const* yi, const double* dyinv, void* hy,
                      int n1, cudaStream_t s) {
   raise_smem_limit<k_slab_upwind_y<UPW, MX>>(200 * 1024);
-  const dim3 grid((P.N0 + TI - 1) / TI, (P.N1 + TJ - 1) / TJ);
+  const dim3 grid = tile_grid(P);
   const size_t smem = (size_t)P.nvars * NY * (MX ? sizeof(float) : sizeof(double));
   k_slab_upwind_y<UPW, MX><<<grid, 256, smem, s>>>(P, UT, yi[0], yi[1], yi[2], yi[3], dyinv, hy, n1);
 }
