@@ -62,7 +62,6 @@ static void free_sim(piafs_gpu_sim* s) {
   cudaFree(s->sponge_buf);
   cudaFree(s->zone_buf);
   cudaFree(s->crwchar);
-  cudaFree(s->fCy);
   if (s->yfork) cudaEventDestroy(s->yfork);
   if (s->yjoin) cudaEventDestroy(s->yjoin);
   if (s->ystream) cudaStreamDestroy(s->ystream);
@@ -422,18 +421,6 @@ int piafs::create_sim(Deck&& deck, int precision, piafs_gpu_sim** out) {
     e = alloc(&s->ut, planes);
     s->PT = transposed_params(P);
   }
-  // The y pass on a stream of its own (2D Navier-Stokes; the characteristic
-  // CRWENO5 solves share one scratch).  PIAFS_GPU_NO_CONCURRENT_Y=1 runs it
-  // after the x pass on one stream (the same values).
-  const char* ncy = std::getenv("PIAFS_GPU_NO_CONCURRENT_Y");
-  if (e == cudaSuccess && P.ndims == 2 && P.model == NS2D && !s->crwchar &&
-      (P.scheme != CRWENO5 || s->ut) && !(ncy && ncy[0] == '1')) {
-    e = alloc(&s->fCy, planes);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->ystream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->yfork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->yjoin, cudaEventDisableTiming);
-    s->concurrent_y = e == cudaSuccess;
-  }
   if (e == cudaSuccess) e = alloc(&s->dxinv, d.dxinv.size());
   if (e == cudaSuccess) e = alloc(&s->imap, d.imap.size());
   if (e == cudaSuccess) e = alloc(&s->tdev, 1);
@@ -443,7 +430,24 @@ int piafs::create_sim(Deck&& deck, int precision, piafs_gpu_sim** out) {
   if (e == cudaSuccess) e = cudaMalloc(&s->err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(s->err, 0, sizeof(int));
   s->aos_bytes = (size_t)P.npg * P.nvars * sizeof(double);
-  if (e == cudaSuccess) e = cudaMalloc(&s->aos, s->aos_bytes);
+  // The y pass on a stream of its own (2D Navier-Stokes; the characteristic
+  // CRWENO5 solves share one scratch).  Its fluxes go into the array that host
+  // transfers are staged in: both are used on the simulation's stream, which a
+  // y pass forks from and joins, so never at once.  (An array of its own was one
+  // state more of device memory: 94 MB of 1.8 GB at 1024^2 with chemistry.)  Without
+  // the stream or an event, and with PIAFS_GPU_NO_CONCURRENT_Y=1, the passes run
+  // in turn (the same values).
+  const char* ncy = std::getenv("PIAFS_GPU_NO_CONCURRENT_Y");
+  const bool ypass = P.ndims == 2 && P.model == NS2D && !s->crwchar && (P.scheme != CRWENO5 || s->ut) &&
+                     !(ncy && ncy[0] == '1');
+  if (e == cudaSuccess) e = cudaMalloc(&s->aos, ypass ? planes * sizeof(double) : s->aos_bytes);
+  if (e == cudaSuccess && ypass) {
+    s->concurrent_y = cudaStreamCreateWithFlags(&s->ystream, cudaStreamNonBlocking) == cudaSuccess &&
+                      cudaEventCreateWithFlags(&s->yfork, cudaEventDisableTiming) == cudaSuccess &&
+                      cudaEventCreateWithFlags(&s->yjoin, cudaEventDisableTiming) == cudaSuccess;
+    if (s->concurrent_y) s->fCy = s->aos;
+    else cudaGetLastError();
+  }
   // the species files carry the photon density of the last RK stage evaluated
   // (zero before the first step, as the reference's calloc'd nv_hnu)
   const bool binary_out = d.op_file_format == "binary" || d.op_file_format == "bin";

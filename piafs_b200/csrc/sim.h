@@ -18,9 +18,9 @@ struct piafs_gpu_sim {
   int precision = 0;
   int device = 0;
   cudaStream_t stream = nullptr;
-  // 2D Navier-Stokes with a transposed y pass: the y pass (transpose, y
-  // flux into fCy, y line solve) on ystream, concurrent with the x pass,
-  // forked from and joined to `stream` by the two events
+  // 2D Navier-Stokes: the y pass (transpose of a transposed one, y flux into
+  // fCy, reconstruction) on ystream, concurrent with the x pass, forked from and
+  // joined to `stream` by the two events; fCy is aos
   bool concurrent_y = false;
   cudaStream_t ystream = nullptr;
   cudaEvent_t yfork = nullptr, yjoin = nullptr;
@@ -48,7 +48,7 @@ struct piafs_gpu_sim {
   double* norm_acc = nullptr;
   unsigned long long* cfl_acc = nullptr;
   int* err = nullptr;
-  double* aos = nullptr;                   // ghosted AoS staging (host transfers)
+  double* aos = nullptr;                   // ghosted AoS staging (host transfers), between them the y fluxes
   size_t aos_bytes = 0;
   double* hnu = nullptr;                   // photon density [nz][ps] of the last RK stage (species output)
   // sponge zones: extents on the host, ramp and reference state in sponge_buf

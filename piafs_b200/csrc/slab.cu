@@ -114,8 +114,7 @@ int piafs_gpu_slab_create(const char* deck_dir, int precision, int rank, int nra
   cudaFree(s->ut);
   s->ut = nullptr;
   s->concurrent_y = false;
-  cudaFree(s->fCy);
-  s->fCy = nullptr;
+  s->fCy = nullptr;   // the staging array, which stays
   for (auto& p : s->iface_y) { cudaFree(p); p = nullptr; }
   // the column slab: columns [rank n0, (rank + 1) n0), every row
   DevParams& C = sl->Pc;
