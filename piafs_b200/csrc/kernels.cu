@@ -1079,9 +1079,6 @@ void launch_soa_to_aos(const double* soa, double* aos, long long npg, int nv, lo
 void launch_soa_to_interior(const DevParams& P, const double* soa, double* out, cudaStream_t s) {
   point_major<false, true>(P, out, const_cast<double*>(soa), (long long)P.N0 * P.N1, P.nvars, P.ps, s);
 }
-void launch_interior_to_soa(const DevParams& P, const double* in, double* soa, cudaStream_t s) {
-  point_major<true, true>(P, const_cast<double*>(in), soa, (long long)P.N0 * P.N1, P.nvars, P.ps, s);
-}
 void launch_iface_aos_to_soa(const double* aos, double* soa, long long ni, int nv, long long pis, cudaStream_t s) {
   point_major<true, false>(DevParams{}, const_cast<double*>(aos), soa, ni, nv, pis, s);
 }

@@ -145,7 +145,6 @@ __device__ __forceinline__ void bc_point(const DevParams& P, const Zone& z, cons
 void launch_aos_to_soa(const double* aos, double* soa, long long npg, int nv, long long ps, cudaStream_t s);
 void launch_soa_to_aos(const double* soa, double* aos, long long npg, int nv, long long ps, cudaStream_t s);
 void launch_soa_to_interior(const DevParams& P, const double* soa, double* out, cudaStream_t s);
-void launch_interior_to_soa(const DevParams& P, const double* in, double* soa, cudaStream_t s);
 void launch_iface_aos_to_soa(const double* aos, double* soa, long long ni, int nv, long long pis, cudaStream_t s);
 void launch_iface_soa_to_aos(const double* soa, double* aos, long long ni, int nv, long long pis, cudaStream_t s);
 // whether the grid is narrower than the ghost layers: a zone's source can then
