@@ -57,7 +57,10 @@ typedef struct {
   long long ninterfaces[2];   /* points of an interface array per dir      */
   double cfl, norm;           /* last diagnostics (TimePreStep/PostStep)   */
   int singular;               /* zero pivots seen since creation           */
-  int launches_per_step;      /* kernels one time step launches            */
+  /* kernels one time step launches; 1 for a 1D Euler line whose steps run
+   * together, up to 1024 to a launch (a step with the residual norm adds a
+   * copy and a small kernel) */
+  int launches_per_step;
 } piafs_gpu_info;
 
 /* Message of the last failure on this thread ("" if none). */
@@ -134,7 +137,10 @@ int piafs_gpu_synchronize(piafs_gpu_sim* sim);
  * y pass), [2d+1] interface reconstruction (WENO5 or the CRWENO5 line
  * solve), then [2 ndims] upwinding + divergence of all directions (in 2D with
  * second-order viscous terms these and the source too, one kernel) and
- * [2 ndims + 1] viscous + source where they are apart, and the sponge zones.  nphases (in/out) is the capacity / count. */
+ * [2 ndims + 1] viscous + source where they are apart, and the sponge zones.
+ * For a 1D Euler line whose steps and right-hand sides are one launch
+ * (launches_per_step 1) these are the phases of its kernel-by-kernel form,
+ * which HyperbolicFunction runs.  nphases (in/out) is the capacity / count. */
 int piafs_gpu_profile_rhs(piafs_gpu_sim* sim, int reps, double* ms, int* nphases);
 
 /* Photon density of the last RK stage evaluated (the reference's

@@ -260,8 +260,8 @@ static void enqueue_step(piafs_gpu_sim* s, bool with_norm) {
   launch_advance_time(s->tdev, d.dt, s->stream);
 }
 
-// Steps of a 1D line in launches of many (bounded, so that no launch runs for
-// longer than some milliseconds).
+// Steps of a 1D line in launches of at most 1024 (7 ms of the 1024-point WENO5
+// line, 44 ms of the 6001-point CRWENO5 one).
 static int enqueue_run1d(piafs_gpu_sim* s, int nsteps) {
   for (int k = 0; k < nsteps;) {
     Run1D R = s->run1d;
@@ -530,7 +530,8 @@ int piafs_gpu_get_info(piafs_gpu_sim* s, piafs_gpu_info* info) {
   info->npoints_ghosted = s->P.npg;
   info->ninterfaces[0] = s->P.nint[0]; info->ninterfaces[1] = s->P.nint[1];
   info->cfl = s->last_cfl; info->norm = s->last_norm; info->singular = s->singular;
-  // kernels per step: the BC launches (nz) of every stage, per stage flux
+  // launches per step: 1 for a 1D line in one launch (which takes up to 1024
+  // steps); else the BC launches (nz) of every stage, per stage flux
   // and reconstruction per direction plus the transpose of a transposed y
   // pass and the upwind / stage kernel, the separate source and combination
   // kernels where they are not part of it, and the clock

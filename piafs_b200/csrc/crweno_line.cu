@@ -21,9 +21,9 @@
 //     and the right-biased row at interface j-1 share (their unnormalised
 //     weights are the same three products with the first and third roles
 //     swapped), so a row pair costs three products instead of six;
-//   * chunks inside the line (every warp but the first and the last) take a
-//     path without any per-row test; only the chunks holding row 1, row N-1
-//     or rows past the line run the general rows;
+//   * chunks inside the line (every warp but the last) take a path without any
+//     per-row test but that of row 1; only the chunks holding row N-1 or rows
+//     past the line run the general rows;
 //   * the PCR rows of both biases are packed as double2, one 16-byte access
 //     per coefficient and neighbour.
 //
@@ -32,9 +32,9 @@
 // computed directly and folded into rows 1 and N-1; rows past N-1 are
 // identity rows.  Every row may be scaled by a positive constant without
 // changing the solution (the elimination normalises each row), which the Jiang-Shu
-// rows use: they are formed at 30x (3x for the compact scheme's thirds, 10x
-// for the optimal weights 0.2, 0.5, 0.3) from unnormalised weights, and the
-// smoothness indicators at 4x with eps at 4x.  Quotients use rcp_nr.
+// rows use: they are formed at 15x (3x for the compact scheme's thirds, 5x
+// for the optimal weights 0.2, 0.5, 0.3 as 1, 5/2, 3/2) from unnormalised weights,
+// and the smoothness indicators at 4x with eps at 4x.  Quotients use rcp_nr.
 #include <cooperative_groups.h>
 #include <type_traits>
 

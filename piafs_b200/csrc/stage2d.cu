@@ -6,16 +6,16 @@
 // combination of the stage (TimeRK.c:60-75, :86-99).  The stage derivative and
 // the next stage's state are written once each, from registers.
 //
-// What bounds it: HBM and its latency.  Of the interface arrays it reads 24
+// What bounds it: HBM and its latency.  Of the interface arrays it reads 26
 // values a point per direction with one chemistry layer and LLF (uL, uR,
-// fL + fR of the four flow variables, uL - uR and fL + fR of the passive
+// fL + fR of the four flow variables, uL - uR and fL + fR of the seven passive
 // ones), and writes 11 (or 22).
 // Separate kernels for the upwinding, the viscous terms and source, and the
 // combination read and wrote the derivative three times over: at 2048^2 with 11
 // variables 0.53 + 0.31 ms and 0.2 ms of combination a stage, where this takes
 // 0.67 ms with the combination; a step of the 512^2 run went from 640 to 574 us,
-// one of 300 x 217 points from 198 to 161 us.  Three CTAs an SM (80 registers)
-// hide the loads; the 16 x 15 tile of the upwinding alone would put 16 points of
+// one of 300 x 217 points from 198 to 161 us.  Three CTAs an SM (80 registers,
+// no spills) hide the loads; the 16 x 15 tile of the upwinding alone would put 16 points of
 // the viscous fluxes in a second round.
 #include <type_traits>
 
