@@ -44,14 +44,17 @@ enum YMode { Y_STD = 0, Y_TRANSPOSED = 1, Y_GIVEN = 2 };
 // 18.4); RF's matrices in FP64 two (1201 x 777: 131.1 us, 133.3 with three).
 constexpr int stage2d_ctas(int upw, bool mx) { return mx ? 4 : upw == UPW_RF ? 2 : 3; }
 
-// The grid of tiles: rows of tiles in y and, past the 65535 a launch takes there,
-// in z (grids of more than 917,490 rows of points).  Tiles that this rounds up to
-// beyond the last row have no interface or point inside the grid.
+// The grid of tiles: rows of tiles in y, ROWS at a time in z (a launch takes 65535
+// in either: grids of 917,491 rows of points and more need both).  Tiles that this
+// rounds up to beyond the last row have no interface or point inside the grid.
+// ROWS is a constant because the row must cost nothing: with the grid's own height
+// in its place the 2048^2 launch took 0.630 ms, with this, or without z, 0.611.
+constexpr int ROWS = 4096;
 dim3 tile_grid(const DevParams& P) {
-  const int tx = (P.N0 + TI - 1) / TI, ty = (P.N1 + TJ - 1) / TJ, nz = (ty + 65534) / 65535;
-  return dim3(tx, (ty + nz - 1) / nz, nz);
+  const int tx = (P.N0 + TI - 1) / TI, ty = (P.N1 + TJ - 1) / TJ;
+  return dim3(tx, ty < ROWS ? ty : ROWS, (ty + ROWS - 1) / ROWS);
 }
-__device__ __forceinline__ int tile_row() { return blockIdx.y + blockIdx.z * gridDim.y; }
+__device__ __forceinline__ int tile_row() { return blockIdx.y + blockIdx.z * ROWS; }
 
 // Threads a CTA.  Up to one tile an SM 512: x and y interfaces by different
 // threads, the chemistry beside the viscous fluxes, a point's variables by two
@@ -84,7 +87,8 @@ constexpr size_t stage2d_smem(int nv, bool given, bool visc) {
 // variables, or 0 for P.nvars; where it is 4 the loop over the passive variables
 // must not be there at all -- room for its loads, never issued, spilled 350 to 370
 // bytes a thread (132 to 136 in mixed precision with a transposed y pass), which
-// cost 0.3 to 1 % of a step at 1201 x 777 (WENO5, Rusanov 668 -> 663 us).
+// cost 0.3 to 1 % of a step at 1201 x 777 (WENO5, Rusanov 668 -> 663 us).  With 11
+// a constant end saves 2 % of the launch (2048^2 0.626 -> 0.611 ms).
 template <int UPW, int DIR, bool MX, int NV>
 __device__ __forceinline__ void iface_upwind(const DevParams& P, const void* __restrict__ uLv,
                                              const void* __restrict__ uRv, const void* __restrict__ fLv,
