@@ -102,6 +102,26 @@ def test_lines(tmp_path, scheme, upw, weno, N, rk, ends):
     check(d, 0.1 / N, rk)
 
 
+@pytest.mark.parametrize("scheme,N", [("weno5", n) for n in (8, 17, 63, 64, 127, 128, 255, 1024, 2047, 4099, 10240, 10241)]
+                         + [("crweno5", n) for n in (16, 255, 256, 257, 258, 513, 1024, 4096, 4098, 4100, 8193, 8194)])
+def test_line_sizes(tmp_path, scheme, N):
+    """Where segments and clusters begin and end (8, 258, 8194 and 10241 points:
+    lines of separate kernels)."""
+    d = str(tmp_path / "l")
+    cases.euler1d_density_wave(d, N=N, n_iter=3, dt=0.1 / N, scheme=scheme)
+    check(d, 0.1 / N, "ssprk3")
+
+
+@pytest.mark.parametrize("scheme", ["weno5", "crweno5"])
+@pytest.mark.parametrize("ends", ["periodic", "walls", "fixed"])
+@pytest.mark.parametrize("rk", ["22", "33", "44", "ssprk3"])
+def test_line_ends(tmp_path, scheme, ends, rk):
+    d = str(tmp_path / "l")
+    cases.euler1d_density_wave(d, N=150, n_iter=3, dt=0.1 / 150, scheme=scheme, time_scheme_type=rk,
+                               weno={"no_limiting": 1} if ends == "periodic" else None, zones=LINE_ENDS[ends])
+    check(d, 0.1 / 150, rk)
+
+
 @pytest.mark.parametrize("rk", ["22", "33", "44", "ssprk3"])
 @pytest.mark.parametrize("layers", [0, 1, 2])
 @pytest.mark.parametrize("N,NY,scheme,upw", [(33, 29, "crweno5", "llf-char"), (200, 230, "weno5", "roe")])
